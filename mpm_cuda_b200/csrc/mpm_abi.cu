@@ -217,7 +217,7 @@ int mpm_kernel_config_scatter(int config, int* cell_major, int* segmented) {
     if (config < 0 || config >= mpm::kNumFusedCfgs)
         return fail(nullptr, MPM_ERR_INVALID, "mpm_kernel_config_scatter: config %d out of range", config);
     if (cell_major) *cell_major = mpm::kFusedCfgs[config].order == mpm::ORDER_CELL ? 1 : 0;
-    if (segmented) *segmented = mpm::kFusedCfgs[config].scatter == mpm::SCATTER_SEGMENTED ? 1 : 0;
+    if (segmented) *segmented = mpm::kFusedCfgs[config].scatter == mpm::SCATTER_RUNS ? 1 : 0;
     return MPM_OK;
 }
 

@@ -8,11 +8,11 @@ namespace mpm {
 // minimum resident CTAs per SM given to __launch_bounds__ (which caps
 // registers at 65536 / (chunk * min_ctas)); scatter: how the P2G of the next
 // substep reaches the grid -- SCATTER_DIRECT: every particle reduces its 3^D
-// node values into global memory (red.global.add.v4.f32); SCATTER_SEGMENTED:
-// the lanes of a warp that share a stencil base (a cell, in cell-major order)
-// are summed in shared memory first and each sum is reduced once (the
-// per-warp staging buffer limits these kernels to fewer CTAs per SM).
-enum : int { SCATTER_DIRECT = 0, SCATTER_SEGMENTED = 1 };
+// node values into global memory (red.global.add.v4.f32); SCATTER_RUNS: the
+// particles of a chunk that share a stencil base are summed first and each
+// sum is reduced once (mpm_kernels_runs.cuh; the chunk's source records in
+// shared memory limit these kernels to fewer CTAs per SM).
+enum : int { SCATTER_DIRECT = 0, SCATTER_RUNS = 1 };
 struct FusedKernel {
     int chunk;
     int min_ctas;
@@ -21,7 +21,7 @@ struct FusedKernel {
 constexpr int kNumFusedKernels = 12;
 constexpr FusedKernel kFusedKernels[kNumFusedKernels] = {
     {128, 4, 0}, {128, 5, 0}, {128, 6, 0}, {64, 8, 0}, {64, 10, 0}, {64, 12, 0}, {256, 2, 0}, {256, 3, 0},
-    {64, 5, 1},  {128, 3, 1}, {64, 4, 1},  {128, 2, 1}};
+    {128, 5, 1}, {128, 4, 1}, {256, 3, 1}, {256, 2, 1}};
 
 // A launch configuration (the autotuner's search space): an instantiation,
 // rounds -- particles each thread processes per chunk, one after the other,
@@ -46,14 +46,14 @@ struct FusedCfgTable {
     static constexpr int N = 36;
     FusedCfg c[N];
     // 0..11 direct scatter, rank-major; 12..23 the same shapes cell-major;
-    // 24..31 segmented scatter (cell-major), one and two rounds; 32..35 the
+    // 24..31 run sums (cell-major), one to three rounds; 32..35 the
     // 64-thread, 10-CTA direct kernel with three and four rounds, rank-major
     // and cell-major (fewer window loads and barrier pairs per particle; on
     // the 2M-particle scenes 3-4 % faster than two rounds)
     constexpr FusedCfgTable() : c{} {
         constexpr int kr[12][2] = {{0, 1}, {1, 1}, {2, 1}, {3, 1}, {4, 1}, {5, 1},
                                    {6, 1}, {7, 1}, {1, 2}, {2, 2}, {4, 2}, {7, 2}};
-        constexpr int sr[8][2] = {{8, 1}, {9, 1}, {10, 1}, {11, 1}, {8, 2}, {9, 2}, {10, 2}, {11, 2}};
+        constexpr int sr[8][2] = {{8, 1}, {8, 2}, {9, 2}, {9, 3}, {10, 1}, {10, 2}, {11, 1}, {11, 2}};
         for (int i = 0; i < 24; ++i) {
             const int k = kr[i % 12][0];
             c[i] = FusedCfg{kFusedKernels[k].chunk, kFusedKernels[k].min_ctas, kr[i % 12][1], k,
@@ -62,7 +62,7 @@ struct FusedCfgTable {
         for (int i = 0; i < 8; ++i) {
             const int k = sr[i][0];
             c[24 + i] = FusedCfg{kFusedKernels[k].chunk, kFusedKernels[k].min_ctas, sr[i][1], k, ORDER_CELL,
-                                 SCATTER_SEGMENTED};
+                                 SCATTER_RUNS};
         }
         for (int i = 0; i < 4; ++i)
             c[32 + i] = FusedCfg{kFusedKernels[4].chunk, kFusedKernels[4].min_ctas, 3 + i % 2, 4,
@@ -75,19 +75,20 @@ constexpr int kNumFusedCfgs = FusedCfgTable::N;
 // fewest particles a chunk of any configuration holds (sizes the chunk lists)
 constexpr int kMinChunkParticles = 64;
 
-// dynamic shared memory of a fused kernel: the segmented scatter's staging
-// buffer, 3^D node values of each of a warp's 32 lanes
-constexpr int seg_rows(int dim) { return dim == 3 ? 27 : 9; }
-constexpr int fused_dyn_smem(int dim, int kernel) {
-    return kFusedKernels[kernel].scatter == SCATTER_SEGMENTED
-               ? kFusedKernels[kernel].chunk / 32 * seg_rows(dim) * 32 * 16
-               : 0;
+// SCATTER_RUNS: float4s of a particle's source record, and the dynamic shared
+// memory of a chunk (a record and a run-list entry per particle)
+constexpr int run_rec4(int dim) { return dim == 3 ? 6 : 4; }
+constexpr int run_smem(int dim, int particles) { return particles * (run_rec4(dim) * 16 + 2); }
+// dynamic shared memory of a launch configuration
+constexpr int fused_dyn_smem(int dim, int cfg) {
+    return kFusedCfgs[cfg].scatter == SCATTER_RUNS ? run_smem(dim, kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds) : 0;
 }
-
-// the direct-scatter instantiation with a kernel's chunk (the learned-stress
-// kernel, which scatters directly, runs with that shape)
-constexpr int direct_kernel_of(int kernel) {
-    return kFusedKernels[kernel].scatter == SCATTER_DIRECT ? kernel : (kFusedKernels[kernel].chunk == 64 ? 3 : 0);
+// the most any configuration of the same instantiation asks for
+constexpr int fused_dyn_smem_max(int dim, int cfg) {
+    int most = 0;
+    for (int i = 0; i < kNumFusedCfgs; ++i)
+        if (kFusedCfgs[i].kernel == kFusedCfgs[cfg].kernel && fused_dyn_smem(dim, i) > most) most = fused_dyn_smem(dim, i);
+    return most;
 }
 
 constexpr bool fused_cfgs_consistent() {
@@ -97,14 +98,10 @@ constexpr bool fused_cfgs_consistent() {
         const FusedKernel& k = kFusedKernels[c.kernel];
         if (k.chunk != c.chunk || k.min_ctas != c.min_ctas || k.scatter != c.scatter ||
             (c.order != ORDER_RANK && c.order != ORDER_CELL) ||
-            (c.scatter == SCATTER_SEGMENTED && c.order != ORDER_CELL) ||
+            (c.scatter == SCATTER_RUNS && c.order != ORDER_CELL) ||
             c.chunk * c.rounds < kMinChunkParticles || c.chunk % 32 != 0)
             return false;
     }
-    for (int k = 0; k < kNumFusedKernels; ++k)
-        if (kFusedKernels[direct_kernel_of(k)].scatter != SCATTER_DIRECT ||
-            kFusedKernels[direct_kernel_of(k)].chunk != kFusedKernels[k].chunk)
-            return false;
     return true;
 }
 static_assert(fused_cfgs_consistent(), "each configuration names the instantiation of its launch shape");

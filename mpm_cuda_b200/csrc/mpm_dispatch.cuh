@@ -4,6 +4,7 @@
 
 #include "mpm_config.cuh"
 #include "mpm_kernels_binned.cuh"
+#include "mpm_kernels_runs.cuh"
 #include "mpm_kernels_surrogate.cuh"
 
 namespace mpm {

@@ -477,7 +477,7 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     update_ctas = (int)std::max<long long>(1, std::min<long long>((total_blocks + 3) / 4, (long long)num_sms * 8));
     cfg = (opt.kernel_config >= 0 && opt.kernel_config < kNumFusedCfgs) ? opt.kernel_config : 1;
     if (paged && kFusedCfgs[cfg].scatter != SCATTER_DIRECT) {
-        msg = "mpm_create: the segmented scatter addresses a dense grid; choose another kernel_config";
+        msg = "mpm_create: the run sums address a dense grid; choose another kernel_config";
         return MPM_ERR_UNSUPPORTED;
     }
     set_config(cfg);
@@ -507,7 +507,7 @@ int Engine::chunk_particles() const { return kFusedCfgs[cfg].chunk * kFusedCfgs[
 
 void Engine::set_config(int ci) {
     cfg = ci;
-    const int dyn = fused_dyn_smem(dim, kFusedCfgs[ci].kernel);
+    const int dyn = fused_dyn_smem(dim, ci);
     for (int mat = 0; mat < kMats; ++mat) {
         int per_sm = 0;
         const FusedFn fn = fused_fn(dim, mat, ci, fixed_scene, paged);
@@ -515,9 +515,12 @@ void Engine::set_config(int ci) {
             fused_ctas[mat] = num_sms;
             continue;
         }
-        // the segmented scatter's staging buffer can exceed the 48 KB a kernel
-        // gets without opting in; a failure here shows in the occupancy query
-        if (dyn > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+        // the source records can exceed the 48 KB a kernel gets without opting
+        // in; a failure here shows in the occupancy query.  The limit is the
+        // function's, shared by every handle: always the most any of its
+        // configurations needs
+        if (dyn > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            fused_dyn_smem_max(dim, ci)) != cudaSuccess)
             cudaGetLastError();
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kFusedCfgs[ci].chunk, dyn) != cudaSuccess) {
             cudaGetLastError();  // the query failed: fall back to one CTA per SM
@@ -562,7 +565,7 @@ namespace {
 struct TuneKey {
     int device, dim, mats;
     long long particles, blocks;
-    bool paged;  // a paged grid has its own kernels (and no segmented scatter)
+    bool paged;  // a paged grid has its own kernels (and no run sums)
     bool operator<(const TuneKey& o) const {
         if (device != o.device) return device < o.device;
         if (dim != o.dim) return dim < o.dim;
@@ -987,7 +990,7 @@ void Engine::enqueue_g2p2g(int parity) {
         } else {
             cudaLaunchAttribute attr;
             const cudaLaunchConfig_t lc = pdl_config(fused_ctas[mat], kFusedCfgs[cfg].chunk,
-                                                     fused_dyn_smem(dim, kFusedCfgs[cfg].kernel), stream, &attr);
+                                                     fused_dyn_smem(dim, cfg), stream, &attr);
             const cudaError_t e = cudaLaunchKernelEx(&lc, fused_fn(dim, mat, cfg, fixed_scene, paged), buf(parity), A);
             note_launch_status("k_g2p2g", e);
             note_launch("fused_fn");

@@ -12,11 +12,13 @@ namespace mpm {
 
 template <int D, int MAT, int K, bool FIXED, bool PAGED>
 static constexpr FusedFn fused_kernel() {
-    if constexpr (PAGED && kFusedKernels[K].scatter == SCATTER_SEGMENTED) {
-        return nullptr;  // the segmented scatter addresses a dense grid
+    constexpr FusedKernel k = kFusedKernels[K];
+    if constexpr (k.scatter == SCATTER_DIRECT) {
+        return &k_g2p2g<D, MAT, k.chunk, k.min_ctas, FIXED, PAGED>;
+    } else if constexpr (!PAGED) {
+        return &k_g2p2g_runs<D, MAT, k.chunk, k.min_ctas, FIXED>;
     } else {
-        return &k_g2p2g<D, MAT, kFusedKernels[K].chunk, kFusedKernels[K].min_ctas, FIXED, kFusedKernels[K].scatter,
-                        PAGED>;
+        return nullptr;  // the run sums address a dense grid
     }
 }
 

@@ -268,6 +268,22 @@ __device__ __forceinline__ bool stencil_paged(const SceneParams& sc, const GridP
     return ok;
 }
 
+// marks the blocks the stencil at `base` covers: it spans at most 2 blocks per
+// axis, so its corner nodes' blocks are all of them
+template <int D>
+__device__ __forceinline__ void mark_stencil(const int* base, const SceneParams& sc, unsigned* blk_flag, int* active,
+                                             int* n_active) {
+#pragma unroll
+    for (int cx = 0; cx < 2; ++cx)
+#pragma unroll
+        for (int cy = 0; cy < 2; ++cy)
+#pragma unroll
+            for (int cz = 0; cz < (D == 3 ? 2 : 1); ++cz) {
+                const int ix = base[0] + 2 * cx, iy = base[1] + 2 * cy, iz = D == 3 ? base[2] + 2 * cz : 0;
+                mark_block(blk_flag, active, n_active, block_of_node<D>(sc, ix, iy, iz));
+            }
+}
+
 // P2G of one particle straight to global memory, marking touched blocks.
 // PAGED: node addresses through the page table; a stencil reaching a block
 // without a page (the pool ran out, or a particle moved more than a cell in a
@@ -289,16 +305,7 @@ __device__ __forceinline__ void p2g_global(const Stencil<D>& st, const P2GSource
             atomicAdd(&g[ix(ox, oy, D == 3 ? oz : 0)], c);
         });
     }
-    // the stencil spans at most 2 blocks per axis: mark its corner blocks
-#pragma unroll
-    for (int cx = 0; cx < 2; ++cx)
-#pragma unroll
-        for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-            for (int cz = 0; cz < (D == 3 ? 2 : 1); ++cz) {
-                const int ix = st.base[0] + 2 * cx, iy = st.base[1] + 2 * cy, iz = D == 3 ? st.base[2] + 2 * cz : 0;
-                mark_block(blk_flag, active, n_active, block_of_node<D>(sc, ix, iy, iz));
-            }
+    mark_stencil<D>(st.base, sc, blk_flag, active, n_active);
 }
 
 // First P2G of a state (after creation or set_state): direct atomics.
@@ -577,29 +584,22 @@ __device__ __forceinline__ void tma_window(const CUtensorMap* map, float4* tv, u
     }
 }
 
-// starts the asynchronous copy of chunk c's grid-velocity window into tv
-// (zero outside the grid), NT threads, and keeps the chunk's record in
-// *s_ch for the chunk's pass.  PAGED: through the page table (zero for a
-// block without a page), and the physical blocks of the window's 3^D blocks
-// (trash outside the scene) into s27 for the chunk's scatter.
+// Starts the asynchronous copy of the grid-velocity window of chunk ch into tv
+// (zero outside the grid), NT threads.  PAGED: through the page table (zero
+// for a block without a page), and the physical blocks of the window's 3^D
+// blocks (trash outside the scene) into s27 for the chunk's scatter.  FIXED
+// dense: one thread issues one box load, completing on `bar`.
 template <int D, int NT, bool FIXED, bool PAGED>
-__device__ __forceinline__ void prefetch_velocity_tile(const FusedArgs& A, int c, float4* tv, int* s27,
-                                                       Chunk* s_ch, unsigned long long* bar) {
+__device__ __forceinline__ void load_window(const FusedArgs& A, const Chunk& ch, float4* tv, int* s27,
+                                            unsigned long long* bar) {
     constexpr int T = TileShape<D>::T;
     constexpr int S = BlockShape<D>::SHIFT;
     constexpr int M = BlockShape<D>::SIDE - 1;
     constexpr int SIDE = BlockShape<D>::SIDE;
     if constexpr (FIXED && !PAGED) {
-        // one box load of the linear velocity tensor, issued by one thread
-        if (threadIdx.x == 0) {
-            const Chunk ch = A.chunks[c];
-            *s_ch = ch;
-            tma_window<D>(&A.vel_map, tv, bar, ch.o);
-        }
+        if (threadIdx.x == 0) tma_window<D>(&A.vel_map, tv, bar, ch.o);
         return;
     }
-    const Chunk ch = A.chunks[c];
-    if (threadIdx.x == 0) *s_ch = ch;
     const SceneParams& sc = chunk_scene<FIXED>(A, ch.scene);
     const float4* g = A.grid_vel + sc.node_off;
     if constexpr (PAGED) {
@@ -634,6 +634,18 @@ __device__ __forceinline__ void prefetch_velocity_tile(const FusedArgs& A, int c
         }
         cp_async16(&tv[tv_idx<D>(tx, ty, tz)], in ? src : A.grid_vel, in);
     }
+}
+
+// the same for chunk c of the list, keeping its record in *s_ch for the
+// chunk's pass
+template <int D, int NT, bool FIXED, bool PAGED>
+__device__ __forceinline__ void prefetch_velocity_tile(const FusedArgs& A, int c, float4* tv, int* s27,
+                                                       Chunk* s_ch, unsigned long long* bar) {
+    if constexpr (FIXED && !PAGED)
+        if (threadIdx.x != 0) return;
+    const Chunk ch = A.chunks[c];
+    if (threadIdx.x == 0) *s_ch = ch;
+    load_window<D, NT, FIXED, PAGED>(A, ch, tv, s27, bar);
 }
 
 // true when the stencil at `base` lies inside the chunk's window
@@ -824,95 +836,6 @@ __device__ __forceinline__ void mark_touched(unsigned touched, const SceneParams
     }
 }
 
-// ---- segmented scatter (SCATTER_SEGMENTED)
-//
-// P2G of a warp's particles with one reduction per (run of lanes sharing a
-// stencil base, node) instead of one per (lane, node).  In cell-major order
-// the particles of a cell are consecutive, so the lanes of a warp form a few
-// runs (about 4 at 8 particles per cell) whose members scatter into the same
-// 3^D nodes.  Each lane writes its 3^D node values to its column of the
-// warp's staging buffer V[row = node][column = lane]; then lane `row` walks
-// the columns in order, summing the values of row `row` over each run, and at
-// a run's last column reduces the sum into that run's node `row` of the grid
-// (red.global.add.v4.f32).  The walk is the same for every lane (run limits
-// are warp-uniform bit masks), so it has no divergence.  Lanes whose stencil
-// left the chunk's window scatter directly to global memory and do not take
-// part; a lane whose base differs from its neighbour's starts a new run, so
-// results do not depend on the order.  Every lane of the warp must call this.
-
-// staging-buffer slot of (row, column): the column XOR-ed with the row's low
-// three bits, so a column write (fixed row, 32 lanes) and a row read (fixed
-// column, one row per lane) both touch distinct 16-byte bank groups
-__device__ __forceinline__ int seg_slot(int row, int col) { return row * 32 + (col ^ (row & 7)); }
-
-template <int D>
-__device__ __forceinline__ void scatter_segmented(bool valid, const Stencil<D>& sn, const P2GSource<D>& src,
-                                                  const SceneParams& sc, const int* o, const FusedArgs& A,
-                                                  unsigned* touched, float4* __restrict__ V) {
-    constexpr int R = seg_rows(D);
-    constexpr int S = BlockShape<D>::SHIFT;
-    constexpr int M = BlockShape<D>::SIDE - 1;
-    constexpr int SIDE = BlockShape<D>::SIDE;
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const bool inw = valid && in_window<D>(sn.base, o);
-    if (valid && !inw) {
-        atomicAdd(A.fallback, 1u);
-        p2g_global<D>(sn, src, sc, A.grid_mom, A.blk_flag, A.active, A.n_active, A.pages, A.err_word);
-    }
-    const unsigned part = __ballot_sync(FULL, inw);
-    if (part == 0u) return;
-    // stencil base in window coordinates (0 .. T - 3 per axis, 4 bits each)
-    const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
-    const int key = inw ? l0 + 16 * (l1 + 16 * l2) : -1;
-    if (inw) {
-        p2g_scatter<D>(sn, src, sc.h, sc.inv_h, [&](int ox, int oy, int oz, float4 c) {
-            V[seg_slot(D == 3 ? (ox * 3 + oy) * 3 + oz : ox * 3 + oy, lane)] = c;
-        });
-    }
-    const int kprev = __shfl_up_sync(FULL, key, 1);
-    const bool head = inw && (lane == 0 || kprev != key);
-    const unsigned heads = __ballot_sync(FULL, head);
-    if (head) atomicOr(touched, touched_bits<D>(l0, l1, l2));
-    const unsigned ends = part & ~((part & ~heads) >> 1);  // the next lane does not continue the run
-    __syncwarp();
-    // this lane's row: stencil node (rx, ry, rz)
-    const int row = lane;
-    const bool has_row = row < R;
-    const int rx = D == 3 ? row / 9 : row / 3, ry = D == 3 ? (row / 3) % 3 : row % 3, rz = D == 3 ? row % 3 : 0;
-    const int px = o[0] + rx, py = o[1] + ry, pz = o[2] + rz;
-    const int sy = sc.nb[0] * 64, sz = sc.nb[0] * sc.nb[1] * 64;
-    float4* g = A.grid_mom + sc.node_off;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int m = 0; m < 32; ++m) {
-        if (!((part >> m) & 1u)) continue;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (has_row) v = V[seg_slot(row, m)];
-        if ((heads >> m) & 1u) {
-            acc = v;
-        } else {
-            acc.x += v.x;
-            acc.y += v.y;
-            acc.z += v.z;
-            acc.w += v.w;
-        }
-        if ((ends >> m) & 1u) {
-            const int km = __shfl_sync(FULL, key, m);
-            if (has_row) {
-                const int gx = px + (km & 15), gy = py + ((km >> 4) & 15);
-                int idx = (gx >> S) * 64 + (gx & M) + (gy >> S) * sy + (gy & M) * SIDE;
-                if (D == 3) {
-                    const int gz = pz + (km >> 8);
-                    idx += (gz >> S) * sz + (gz & M) * SIDE * SIDE;
-                }
-                atomicAdd(&g[idx], acc);
-            }
-        }
-    }
-    __syncwarp();  // the buffer is rewritten by the next call
-}
-
 // Per-CTA maximum of the particles' signal speed |v| + wave for adaptive dt:
 // warps reduce into a shared word during a chunk, thread 0 folds it into a
 // running maximum of the current scene after the chunk and sends one global
@@ -1022,21 +945,18 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
 // and InterpolateAndMove as three kernels with full-grid sweeps and host
 // syncs between them).  The P2G scatter reduces into global memory with
 // float4 vector reductions (red.global.add.v4.f32), per particle
-// (SCATTER_DIRECT) or per run of a warp's lanes sharing a stencil base
-// (SCATTER_SEGMENTED, staging buffer in dynamic shared memory).  FIXED: the
-// scene comes from A.scene (one scene, dt fixed for the run).
-template <int D, int MAT, int CHUNK, int MINB, bool FIXED, int SCATTER, bool PAGED>
+// (SCATTER_DIRECT; mpm_kernels_runs.cuh sums the particles that share a
+// stencil base first).  FIXED: the scene comes from A.scene (one scene, dt
+// fixed for the run).
+template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
     using P = Planes<D>;
     using TS = TileShape<D>;
-    static_assert(!(PAGED && SCATTER == SCATTER_SEGMENTED), "the segmented scatter addresses a dense grid");
     __shared__ __align__(128) float4 tv[2][TS::VN];  // grid velocity windows (double-buffered; box-load targets)
     __shared__ int s27[2][27];                      // PAGED: the windows' physical blocks
     __shared__ unsigned touched[2];                 // 3^D neighbour-block bits
     __shared__ int s_cn[2];
     __shared__ unsigned s_speed;                    // adaptive dt: this chunk's max signal speed
-    extern __shared__ __align__(16) float4 seg_stage[];  // SCATTER_SEGMENTED: per-warp staging buffers
-    float4* V = seg_stage + (threadIdx.x >> 5) * (seg_rows(D) * 32);
 
     pdl_wait();     // the grid update ahead of this launch has finished
     pdl_trigger();  // the next pass may launch; it waits for this one to end
@@ -1050,13 +970,6 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
 #pragma unroll 1
         for (int r = 0; r < A.rounds; ++r) {
             const int li = (int)threadIdx.x + r * CHUNK;  // this round's particle of the chunk
-            // SCATTER_SEGMENTED: sn and src are scattered after the particle's
-            // branch, by every lane of the warp together; SCATTER_DIRECT
-            // scatters inside it (fewer live registers across the branch)
-            bool scatter = false;
-            Stencil<D> sn;
-            P2GSource<D> src;
-            if constexpr (SCATTER == SCATTER_SEGMENTED) sn.base[0] = sn.base[1] = sn.base[2] = 0;
             if (li < ch.count) {
                 const long long i = (long long)ch.start + li;
                 float* S = pb.s;
@@ -1078,16 +991,16 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
                     if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
 
                     // ---- stress + P2G of the next substep (its dt is dt_next)
+                    Stencil<D> sn;
                     if (make_stencil<D>(x, sc, sn, err)) {
+                        P2GSource<D> src;
                         if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
                         else particle_stress_source<D, MAT>(v, Cn, F, aux, g, sc.dt_next, src);
-                        if constexpr (SCATTER == SCATTER_SEGMENTED) scatter = true;
-                        else scatter_global<D, PAGED>(sn, src, sc, o, A, tb, wpages);
+                        scatter_global<D, PAGED>(sn, src, sc, o, A, tb, wpages);
                     }
                 }
                 if (err) atomicOr(A.err_word, err);
             }
-            if constexpr (SCATTER == SCATTER_SEGMENTED) scatter_segmented<D>(scatter, sn, src, sc, o, A, tb, V);
         }
         if (A.speed_max) speed_warp_reduce(speed_bits, &s_speed);
     }, [&](int si) { speed.fold(si, &s_speed, A.speed_max); });

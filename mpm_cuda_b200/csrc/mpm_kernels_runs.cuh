@@ -1,0 +1,350 @@
+// Fused substep whose P2G sums the particles that share a stencil base before
+// it reduces into the grid (SCATTER_RUNS).  Same pass as k_g2p2g, in two
+// phases per chunk:
+//   A. every thread: G2P, update and stress of its particles; each particle's
+//      P2G source goes to a record in shared memory and onto the list of the
+//      records with its base node (a run: one exchange on the base's head);
+//   B. a thread per (run, x-plane of the stencil): walks the run's records,
+//      sums its nine nodes in registers and reduces each once.
+// k_g2p2g is bound by the L1 data pipe and the L1-to-L2 request path (66 % busy
+// each on the 2M-particle jello scene): a float4 reduction instruction takes 26
+// data wavefronts, and it issues 27 per particle.  Here a run's particles share
+// its 27 reductions (39.3M -> 6.3M reduction sectors per launch; data pipe 48 %,
+// request path 25 %), for 19 % more instructions; the pass is bound by
+// instruction issue (63 % of the issue slots).  Fused pass, 128 threads x 2
+// particles against the best direct configuration: jello 256^3 2M particles 248
+// against 322 us, snow 256^3 264 against 311, jello 128^3 70 against 88, water
+// 149 x 122 x 83 600k particles 71 against 101, 16 mixed scenes 294 against 364.
+// The records stay in the order of the particles: linking them per base (one
+// exchange each) needs no sort, and a drifted particle joins its new base's run.
+#pragma once
+
+#include "mpm_kernels_binned.cuh"
+
+namespace mpm {
+
+// bases a stencil inside the window can have, per axis and in all
+template <int D>
+struct RunShape {
+    static constexpr int B = TileShape<D>::T - 2;
+    static constexpr int N = D == 3 ? B * B * B : B * B;
+    static constexpr int PLANES = D == 3 ? 3 : 1;  // threads per run
+};
+// run-list entry of a particle whose stencil left the window: this bit and its slot
+constexpr unsigned kRunOutside = 0x8000u;
+
+__device__ __forceinline__ float2 dup2(float s) { return make_float2(s, s); }
+
+// A particle's source record: with alpha = m v - h (m C) f, beta = h m C and
+// A' = A / h (p2g_scatter), columns of beta and the symmetric A' as
+//   3D  (alpha, m) (beta_0, fx) (beta_1, fy) (beta_2, fz)
+//       (A'00, A'01, A'01, A'11) (A'02, A'12, A'22, next)
+//   2D  (alpha, m, next) (beta_0, beta_1) (A'00, A'01, A'01, A'11) (fx, fy)
+template <int D>
+__device__ __forceinline__ void write_record(float4* __restrict__ r, const Stencil<D>& st, const P2GSource<D>& src,
+                                             float h, float inv_h, int next) {
+    float alpha[D], beta[D][D], Ap[D][D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        float a0 = src.mv[c];
+#pragma unroll
+        for (int b = 0; b < D; ++b) {
+            a0 = fmaf(-h * src.mC[c * D + b], st.fx[b], a0);
+            beta[c][b] = h * src.mC[c * D + b];
+            Ap[c][b] = inv_h * src.A[c * D + b];
+        }
+        alpha[c] = a0;
+    }
+    if constexpr (D == 3) {
+        r[0] = make_float4(alpha[0], alpha[1], alpha[2], src.m);
+        r[1] = make_float4(beta[0][0], beta[1][0], beta[2][0], st.fx[0]);
+        r[2] = make_float4(beta[0][1], beta[1][1], beta[2][1], st.fx[1]);
+        r[3] = make_float4(beta[0][2], beta[1][2], beta[2][2], st.fx[2]);
+        r[4] = make_float4(Ap[0][0], Ap[0][1], Ap[0][1], Ap[1][1]);
+        r[5] = make_float4(Ap[0][2], Ap[1][2], Ap[2][2], __int_as_float(next));
+    } else {
+        r[0] = make_float4(alpha[0], alpha[1], src.m, __int_as_float(next));
+        r[1] = make_float4(beta[0][0], beta[1][0], beta[0][1], beta[1][1]);
+        r[2] = make_float4(Ap[0][0], Ap[0][1], Ap[0][1], Ap[1][1]);
+        r[3] = make_float4(st.fx[0], st.fx[1], 0.f, 0.f);
+    }
+}
+
+// Sums of one run over the nine nodes (oy, oz) of stencil plane ox (3D; the
+// nodes (ox, oy) in 2D).  With per-plane vectors
+//   a = wx (alpha + ox beta_0) + dx A'_0, b = wx beta_1, c = wx beta_2,
+//   e = wx A'_1, g = wx A'_2
+// node (oy, oz) gets wz (U + oz V) + dz W, U = wy (a + oy b) + dy e,
+// V = wy c, W = wy g: the contraction of p2g_scatter, x taken first.
+struct PlaneSums {
+    float2 xy[9];
+    float z[9], m[9];
+};
+
+__device__ __forceinline__ void axis3(float f, float (&w)[3], float (&d)[3]) {
+    const float t0 = 1.5f - f, t1 = f - 1.f, t2 = f - 0.5f;
+    w[0] = 0.5f * t0 * t0;
+    w[1] = 0.75f - t1 * t1;
+    w[2] = 0.5f * t2 * t2;
+    d[0] = -t0;
+    d[1] = -2.f * t1;
+    d[2] = t2;
+}
+
+__device__ __forceinline__ void sum_plane3(const float4* __restrict__ recs, int slot, int ox, PlaneSums& acc) {
+    // wx(ox) = s t^2 + k, wx' = 2 s t, t = fx - c
+    const float c = 1.5f - 0.5f * (float)ox, s = ox == 1 ? -1.f : 0.5f, k = ox == 1 ? 0.75f : 0.f;
+    const float2 o2 = dup2((float)ox);
+#pragma unroll
+    for (int n = 0; n < 9; ++n) {
+        acc.xy[n] = make_float2(0.f, 0.f);
+        acc.z[n] = acc.m[n] = 0.f;
+    }
+    do {
+        const float4* r = recs + slot * run_rec4(3);
+        const float4 q5 = r[5], q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3], q4 = r[4];
+        slot = __float_as_int(q5.w);
+        const float t = q1.w - c, st = s * t, wx = fmaf(st, t, k), dx = st + st;
+        const float2 wx2 = dup2(wx);
+        const float2 a = __ffma2_rn(wx2, __ffma2_rn(o2, make_float2(q1.x, q1.y), make_float2(q0.x, q0.y)),
+                                    __fmul2_rn(dup2(dx), make_float2(q4.x, q4.y)));
+        const float a_z = fmaf(wx, fmaf(o2.x, q1.z, q0.z), dx * q5.x);
+        const float2 b = __fmul2_rn(wx2, make_float2(q2.x, q2.y)), cc = __fmul2_rn(wx2, make_float2(q3.x, q3.y));
+        const float2 e = __fmul2_rn(wx2, make_float2(q4.z, q4.w)), g = __fmul2_rn(wx2, make_float2(q5.x, q5.y));
+        const float b_z = wx * q2.z, c_z = wx * q3.z, e_z = wx * q5.y, g_z = wx * q5.z, mw = wx * q0.w;
+        float wy[3], dy[3], wz[3], dz[3];
+        axis3(q2.w, wy, dy);
+        axis3(q3.w, wz, dz);
+#pragma unroll
+        for (int oy = 0; oy < 3; ++oy) {
+            const float2 wy2 = dup2(wy[oy]);
+            float2 U = __ffma2_rn(wy2, a, __fmul2_rn(dup2(dy[oy]), e));
+            float U_z = fmaf(wy[oy], a_z, dy[oy] * e_z);
+            if (oy > 0) {
+                const float wo = (float)oy * wy[oy];
+                U = __ffma2_rn(dup2(wo), b, U);
+                U_z = fmaf(wo, b_z, U_z);
+            }
+            const float2 V = __fmul2_rn(wy2, cc), W = __fmul2_rn(wy2, g);
+            const float V_z = wy[oy] * c_z, W_z = wy[oy] * g_z, M = mw * wy[oy];
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) {
+                if (oz > 0) {
+                    U = __fadd2_rn(U, V);
+                    U_z += V_z;
+                }
+                const int n = oy * 3 + oz;
+                acc.xy[n] = __ffma2_rn(dup2(wz[oz]), U, __ffma2_rn(dup2(dz[oz]), W, acc.xy[n]));
+                acc.z[n] = fmaf(wz[oz], U_z, fmaf(dz[oz], W_z, acc.z[n]));
+                acc.m[n] = fmaf(wz[oz], M, acc.m[n]);
+            }
+        }
+    } while (slot >= 0);
+}
+
+__device__ __forceinline__ void sum_plane2(const float4* __restrict__ recs, int slot, PlaneSums& acc) {
+#pragma unroll
+    for (int n = 0; n < 9; ++n) {
+        acc.xy[n] = make_float2(0.f, 0.f);
+        acc.z[n] = acc.m[n] = 0.f;
+    }
+    do {
+        const float4* r = recs + slot * run_rec4(2);
+        const float4 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3];
+        slot = __float_as_int(q0.w);
+        float wx[3], dx[3], wy[3], dy[3];
+        axis3(q3.x, wx, dx);
+        axis3(q3.y, wy, dy);
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+            float2 a = make_float2(q0.x, q0.y);
+            if (ox > 0) a = __ffma2_rn(dup2((float)ox), make_float2(q1.x, q1.y), a);
+            a = __ffma2_rn(dup2(wx[ox]), a, __fmul2_rn(dup2(dx[ox]), make_float2(q2.x, q2.y)));
+            const float2 b = __fmul2_rn(dup2(wx[ox]), make_float2(q1.z, q1.w));
+            const float2 e = __fmul2_rn(dup2(wx[ox]), make_float2(q2.z, q2.w));
+            const float mw = q0.z * wx[ox];
+#pragma unroll
+            for (int oy = 0; oy < 3; ++oy) {
+                const int n = ox * 3 + oy;
+                if (oy > 0) a = __fadd2_rn(a, b);
+                acc.xy[n] = __ffma2_rn(dup2(wy[oy]), a, __ffma2_rn(dup2(dy[oy]), e, acc.xy[n]));
+                acc.m[n] = fmaf(wy[oy], mw, acc.m[n]);
+            }
+        }
+    } while (slot >= 0);
+}
+
+template <int D, int MAT, int CHUNK, int MINB, bool FIXED>
+__global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
+    using P = Planes<D>;
+    using TS = TileShape<D>;
+    using RS = RunShape<D>;
+    constexpr bool TMA = FIXED;
+    __shared__ __align__(128) float4 tv[TS::VN];  // the chunk's velocity window
+    __shared__ int head[2][RS::N];                // first record of each base's run, -1: none
+    __shared__ int n_runs[2];
+    __shared__ unsigned touched[2];               // 3^D neighbour-block bits
+    __shared__ int s_next[2];
+    __shared__ __align__(16) Chunk s_ch[2];
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ unsigned s_speed;                  // adaptive dt: this chunk's max signal speed
+    extern __shared__ __align__(16) float4 recs[];
+    unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
+
+    for (int t = threadIdx.x; t < 2 * RS::N; t += CHUNK) head[t / RS::N][t % RS::N] = -1;
+    if (threadIdx.x < 2) {
+        n_runs[threadIdx.x] = 0;
+        touched[threadIdx.x] = 0u;
+    }
+    if (threadIdx.x == 0) {
+        s_speed = 0u;
+        if constexpr (TMA) {
+            mbar_init(&s_bar);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+    }
+    pdl_wait();     // the grid update ahead of this launch has finished
+    pdl_trigger();  // the next pass may launch; it waits for this one to end
+    if (A.bump_epoch && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.epoch, 1);
+    const int nch = *A.n_chunks;
+    // the first chunk is the CTA's own index, later ones come from the cursor
+    int cur = blockIdx.x;
+    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, false>(A, cur, tv, nullptr, &s_ch[0], &s_bar);
+    cp_async_commit();
+    SpeedFlush speed;
+    __syncthreads();  // s_bar and the lists initialised
+    for (int k = 0; cur < nch; ++k) {
+        const int b = k & 1;
+        int nxt = 0;
+        if (threadIdx.x == 0) nxt = (int)gridDim.x + atomicAdd(A.cursor, 1);
+        cp_async_wait<0>();
+        // (1) the window and the chunk's record are there; the last chunk's runs are summed
+        if constexpr (TMA) {
+            const bool ok = mbar_wait(&s_bar, (unsigned)k & 1u);
+            if (__syncthreads_or(!ok)) {  // a window that never arrived: report it and stop
+                if (threadIdx.x == 0) atomicOr(A.err_word, ERR_TIMEOUT);
+                break;
+            }
+        } else {
+            __syncthreads();
+        }
+        const Chunk ch = s_ch[b];
+        const SceneParams& sc = chunk_scene<FIXED>(A, ch.scene);
+        const int o[3] = {ch.o[0], ch.o[1], ch.o[2]};
+        unsigned speed_bits = 0u;
+#pragma unroll 1
+        for (int r = 0; r < A.rounds; ++r) {
+            const int li = (int)threadIdx.x + r * CHUNK;  // this round's particle of the chunk
+            if (li < ch.count) {
+                const long long i = (long long)ch.start + li;
+                float* S = pb.s;
+                const long long cap = pb.cap;
+                unsigned err = 0;
+                float x[D];
+#pragma unroll
+                for (int a = 0; a < D; ++a) x[a] = S[(P::X + a) * cap + i];
+                Stencil<D> st;
+                if (make_stencil<D>(x, sc, st, err)) {
+                    G2PAcc<D> acc;
+                    g2p_window<D, false, FIXED>(st, o, tv, sc, A, acc);
+                    // loaded after the gather, its register peak
+                    const GroupParams g = particle_group<FIXED>(A, pb, i);
+                    float F[D * D], Cn[D * D], v[D], aux;
+                    ElasticSVD<D> esvd;
+                    err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux,
+                                                    MAT == SNOW ? &esvd : nullptr, A.defer_vc != 0);
+                    if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
+                    Stencil<D> sn;
+                    if (make_stencil<D>(x, sc, sn, err)) {
+                        P2GSource<D> src;
+                        if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
+                        else particle_stress_source<D, MAT>(v, Cn, F, aux, g, sc.dt_next, src);
+                        int next = -1;
+                        if (in_window<D>(sn.base, o)) {
+                            const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
+                            const int key = l0 + RS::B * (l1 + RS::B * l2);
+                            next = atomicExch(&head[b][key], li);
+                            if (next < 0) {
+                                runs[atomicAdd(&n_runs[b], 1)] = (unsigned short)key;
+                                atomicOr(&touched[b], touched_bits<D>(l0, l1, l2));
+                            }
+                        } else {
+                            atomicAdd(A.fallback, 1u);
+                            runs[atomicAdd(&n_runs[b], 1)] = (unsigned short)(kRunOutside | (unsigned)li);
+                        }
+                        write_record<D>(recs + li * run_rec4(D), sn, src, sc.h, sc.inv_h, next);
+                    }
+                }
+                if (err) atomicOr(A.err_word, err);
+            }
+            // the next chunk's record, on its way while the rest of this phase runs
+            if (r == 0 && threadIdx.x == 0 && nxt < nch) {
+                cp_async16(&s_ch[b ^ 1], &A.chunks[nxt], true);
+                cp_async16(reinterpret_cast<char*>(&s_ch[b ^ 1]) + 16, reinterpret_cast<const char*>(&A.chunks[nxt]) + 16,
+                           true);
+            }
+        }
+        if (A.speed_max) speed_warp_reduce(speed_bits, &s_speed);
+        if (threadIdx.x == 0) {
+            s_next[b] = nxt;
+            cp_async_commit();
+            cp_async_wait<0>();
+        }
+        __syncthreads();  // (2) records, runs and the next chunk's record complete; the window is free
+        const int next_chunk = s_next[b];
+        if (next_chunk < nch) load_window<D, CHUNK, FIXED, false>(A, s_ch[b ^ 1], tv, nullptr, &s_bar);
+        cp_async_commit();
+        mark_touched<D>(touched[b], sc, o, A);
+        speed.fold(ch.scene, &s_speed, A.speed_max);
+        // the other parity's lists were last read before barrier (1)
+        for (int t = threadIdx.x; t < RS::N; t += CHUNK) head[b ^ 1][t] = -1;
+        if (threadIdx.x == 0) {
+            n_runs[b ^ 1] = 0;
+            touched[b ^ 1] = 0u;
+        }
+        // ---- phase B
+        const int items = n_runs[b] * RS::PLANES;
+        for (int it = threadIdx.x; it < items; it += CHUNK) {
+            const int run = D == 3 ? it / 3 : it, ox = D == 3 ? it - 3 * run : 0;
+            const unsigned e = runs[run];
+            int base[3] = {o[0], o[1], o[2]};
+            int slot;
+            if (e & kRunOutside) {
+                // a particle that drifted out of the window: a run of its own,
+                // its base from the position this CTA has just stored
+                slot = (int)(e & (kRunOutside - 1u));
+                float x[D];
+#pragma unroll
+                for (int a = 0; a < D; ++a) x[a] = pb.s[(P::X + a) * pb.cap + ch.start + slot];
+                Stencil<D> sn;
+                unsigned err = 0;
+                make_stencil<D>(x, sc, sn, err);
+#pragma unroll
+                for (int a = 0; a < D; ++a) base[a] = sn.base[a];
+                if (ox == 0) mark_stencil<D>(base, sc, A.blk_flag, A.active, A.n_active);
+            } else {
+                slot = head[b][e];
+                const int l12 = (int)e / RS::B;
+                base[0] += (int)e - RS::B * l12;
+                base[1] += D == 3 ? l12 % RS::B : l12;
+                if (D == 3) base[2] += l12 / RS::B;
+            }
+            PlaneSums acc;
+            if constexpr (D == 3) sum_plane3(recs, slot, ox, acc);
+            else sum_plane2(recs, slot, acc);
+            const StencilIndex<D> ix(sc, base);
+            float4* gm = A.grid_mom + sc.node_off;
+#pragma unroll
+            for (int n = 0; n < 9; ++n) {
+                int at;
+                if constexpr (D == 3) at = (ox == 0 ? ix.x[0] : ox == 1 ? ix.x[1] : ix.x[2]) + ix.y[n / 3] + ix.z[n % 3];
+                else at = ix(n / 3, n % 3, 0);
+                atomicAdd(&gm[at], make_float4(acc.xy[n].x, acc.xy[n].y, acc.z[n], acc.m[n]));
+            }
+        }
+        cur = next_chunk;
+    }
+    speed.flush(A.speed_max);
+}
+
+}  // namespace mpm
