@@ -21,7 +21,7 @@ struct FusedKernel {
 constexpr int kNumFusedKernels = 12;
 constexpr FusedKernel kFusedKernels[kNumFusedKernels] = {
     {128, 4, 0}, {128, 5, 0}, {128, 6, 0}, {64, 8, 0}, {64, 10, 0}, {64, 12, 0}, {256, 2, 0}, {256, 3, 0},
-    {128, 5, 1}, {128, 4, 1}, {256, 3, 1}, {256, 2, 1}};
+    {128, 5, 1}, {128, 4, 1}, {64, 9, 1}, {64, 7, 1}};
 
 // A launch configuration (the autotuner's search space): an instantiation,
 // rounds -- particles each thread processes per chunk, one after the other,
@@ -46,14 +46,17 @@ struct FusedCfgTable {
     static constexpr int N = 36;
     FusedCfg c[N];
     // 0..11 direct scatter, rank-major; 12..23 the same shapes cell-major;
-    // 24..31 run sums (cell-major), one to three rounds; 32..35 the
+    // 24..31 run sums (cell-major), one to three rounds: two rounds of the
+    // 128-thread kernel are the fastest from 400k particles up (256 particles
+    // a chunk: about five per run), one round below, where the chunks are too
+    // few to fill the SMs; 32..35 the
     // 64-thread, 10-CTA direct kernel with three and four rounds, rank-major
     // and cell-major (fewer window loads and barrier pairs per particle; on
     // the 2M-particle scenes 3-4 % faster than two rounds)
     constexpr FusedCfgTable() : c{} {
         constexpr int kr[12][2] = {{0, 1}, {1, 1}, {2, 1}, {3, 1}, {4, 1}, {5, 1},
                                    {6, 1}, {7, 1}, {1, 2}, {2, 2}, {4, 2}, {7, 2}};
-        constexpr int sr[8][2] = {{8, 1}, {8, 2}, {9, 2}, {9, 3}, {10, 1}, {10, 2}, {11, 1}, {11, 2}};
+        constexpr int sr[8][2] = {{8, 1}, {8, 2}, {9, 1}, {9, 2}, {9, 3}, {10, 1}, {11, 1}, {11, 2}};
         for (int i = 0; i < 24; ++i) {
             const int k = kr[i % 12][0];
             c[i] = FusedCfg{kFusedKernels[k].chunk, kFusedKernels[k].min_ctas, kr[i % 12][1], k,
@@ -75,6 +78,8 @@ constexpr int kNumFusedCfgs = FusedCfgTable::N;
 // fewest particles a chunk of any configuration holds (sizes the chunk lists)
 constexpr int kMinChunkParticles = 64;
 
+// particles per thread of a run-sum chunk at most
+constexpr int kMaxRunRounds = 3;
 // SCATTER_RUNS: float4s of a particle's source record, and the dynamic shared
 // memory of a chunk (a record and a run-list entry per particle)
 constexpr int run_rec4(int dim) { return dim == 3 ? 6 : 4; }
@@ -99,7 +104,8 @@ constexpr bool fused_cfgs_consistent() {
         if (k.chunk != c.chunk || k.min_ctas != c.min_ctas || k.scatter != c.scatter ||
             (c.order != ORDER_RANK && c.order != ORDER_CELL) ||
             (c.scatter == SCATTER_RUNS && c.order != ORDER_CELL) ||
-            c.chunk * c.rounds < kMinChunkParticles || c.chunk % 32 != 0)
+            (c.scatter == SCATTER_RUNS && c.rounds > kMaxRunRounds) || c.chunk * c.rounds < kMinChunkParticles ||
+            c.chunk % 32 != 0)
             return false;
     }
     return true;

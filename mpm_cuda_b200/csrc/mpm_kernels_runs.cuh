@@ -17,6 +17,11 @@
 // 149 x 122 x 83 600k particles 71 against 101, 16 mixed scenes 294 against 364.
 // The records stay in the order of the particles: linking them per base (one
 // exchange each) needs no sort, and a drifted particle joins its new base's run.
+// Ordering the runs by length (a counting sort over 16 lengths, two barriers)
+// keeps a warp's lanes on runs of about one length: 248 -> 239 us, jello 128^3
+// 70.5 -> 67.7 us.  Letting a warp start on the next chunk before the others
+// have summed their runs (the first barrier moved to the first record) was
+// slower: the values live across it spill (213 -> 217 us with the Newton stress).
 #pragma once
 
 #include "mpm_kernels_binned.cuh"
@@ -32,6 +37,8 @@ struct RunShape {
 };
 // run-list entry of a particle whose stencil left the window: this bit and its slot
 constexpr unsigned kRunOutside = 0x8000u;
+// runs are ordered by length, those of kRunBins or more together
+constexpr int kRunBins = 16;
 
 __device__ __forceinline__ float2 dup2(float s) { return make_float2(s, s); }
 
@@ -182,7 +189,9 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
     constexpr bool TMA = FIXED;
     __shared__ __align__(128) float4 tv[TS::VN];  // the chunk's velocity window
     __shared__ int head[2][RS::N];                // first record of each base's run, -1: none
+    __shared__ int cnt[2][RS::N];                 // its length
     __shared__ int n_runs[2];
+    __shared__ __align__(16) int hist[kRunBins];  // runs per length, longest first
     __shared__ unsigned touched[2];               // 3^D neighbour-block bits
     __shared__ int s_next[2];
     __shared__ __align__(16) Chunk s_ch[2];
@@ -191,7 +200,11 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
     extern __shared__ __align__(16) float4 recs[];
     unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
 
-    for (int t = threadIdx.x; t < 2 * RS::N; t += CHUNK) head[t / RS::N][t % RS::N] = -1;
+    for (int t = threadIdx.x; t < 2 * RS::N; t += CHUNK) {
+        (&head[0][0])[t] = -1;
+        (&cnt[0][0])[t] = 0;
+    }
+    if (threadIdx.x < kRunBins) hist[threadIdx.x] = 0;
     if (threadIdx.x < 2) {
         n_runs[threadIdx.x] = 0;
         touched[threadIdx.x] = 0u;
@@ -264,6 +277,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
                             const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
                             const int key = l0 + RS::B * (l1 + RS::B * l2);
                             next = atomicExch(&head[b][key], li);
+                            atomicAdd(&cnt[b][key], 1);
                             if (next < 0) {
                                 runs[atomicAdd(&n_runs[b], 1)] = (unsigned short)key;
                                 atomicOr(&touched[b], touched_bits<D>(l0, l1, l2));
@@ -279,9 +293,10 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
             }
             // the next chunk's record, on its way while the rest of this phase runs
             if (r == 0 && threadIdx.x == 0 && nxt < nch) {
-                cp_async16(&s_ch[b ^ 1], &A.chunks[nxt], true);
-                cp_async16(reinterpret_cast<char*>(&s_ch[b ^ 1]) + 16, reinterpret_cast<const char*>(&A.chunks[nxt]) + 16,
-                           true);
+                const char* from = reinterpret_cast<const char*>(&A.chunks[nxt]);
+                char* to = reinterpret_cast<char*>(&s_ch[b ^ 1]);
+                cp_async16(to, from, true);
+                cp_async16(to + 16, from + 16, true);
             }
         }
         if (A.speed_max) speed_warp_reduce(speed_bits, &s_speed);
@@ -297,13 +312,43 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         mark_touched<D>(touched[b], sc, o, A);
         speed.fold(ch.scene, &s_speed, A.speed_max);
         // the other parity's lists were last read before barrier (1)
-        for (int t = threadIdx.x; t < RS::N; t += CHUNK) head[b ^ 1][t] = -1;
+        for (int t = threadIdx.x; t < RS::N; t += CHUNK) {
+            head[b ^ 1][t] = -1;
+            cnt[b ^ 1][t] = 0;
+        }
         if (threadIdx.x == 0) {
             n_runs[b ^ 1] = 0;
             touched[b ^ 1] = 0u;
         }
+        // the runs by length, the longest first, so that the lanes of a warp
+        // walk runs of about one length: a run's place is the number of longer
+        // runs plus its rank among those of its length
+        const int nr = n_runs[b];
+        unsigned entry[kMaxRunRounds];
+        int bin[kMaxRunRounds], rank[kMaxRunRounds];
+#pragma unroll
+        for (int q = 0; q < kMaxRunRounds; ++q) {
+            const int t = (int)threadIdx.x + q * CHUNK;
+            if (t < nr) {
+                entry[q] = runs[t];
+                const int len = (entry[q] & kRunOutside) ? 1 : cnt[b][entry[q]];
+                bin[q] = kRunBins - min(len, kRunBins);
+                rank[q] = atomicAdd(&hist[bin[q]], 1);
+            }
+        }
+        __syncthreads();  // (3)
+#pragma unroll
+        for (int q = 0; q < kMaxRunRounds; ++q) {
+            if ((int)threadIdx.x + q * CHUNK < nr) {
+                int at = rank[q];
+                for (int j = 0; j < bin[q]; ++j) at += hist[j];
+                runs[at] = (unsigned short)entry[q];
+            }
+        }
+        __syncthreads();  // (4)
+        if (threadIdx.x < kRunBins) hist[threadIdx.x] = 0;
         // ---- phase B
-        const int items = n_runs[b] * RS::PLANES;
+        const int items = nr * RS::PLANES;
         for (int it = threadIdx.x; it < items; it += CHUNK) {
             const int run = D == 3 ? it / 3 : it, ox = D == 3 ? it - 3 * run : 0;
             const unsigned e = runs[run];
