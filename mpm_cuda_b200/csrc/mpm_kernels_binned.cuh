@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128) k_p2g_prologue(ParticleBuf pb, long long 
         return;
     }
     P2GSource<D> src;
-    particle_stress_source<D>(v, C, F, aux, g, sc, src);
+    particle_stress_source<D, -1, true>(v, C, F, aux, g, sc, src);
     p2g_global<D, PAGED>(st, src, sc, grid_mom, blk_flag, active, n_active, gp, err_word);
 }
 
@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
                     if (make_stencil<D>(x, sc, sn, err)) {
                         P2GSource<D> src;
                         if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
-                        else particle_stress_source<D, MAT>(v, Cn, F, aux, g, sc.dt_next, src);
+                        else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
                         scatter_global<D, PAGED>(sn, src, sc, o, A, tb, wpages);
                     }
                 }

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
                     if (make_stencil<D>(x, sc, sn, err)) {
                         P2GSource<D> src;
                         if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
-                        else particle_stress_source<D, MAT>(v, Cn, F, aux, g, sc.dt_next, src);
+                        else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
                         int next = -1;
                         if (in_window<D>(sn.base, o)) {
                             const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;

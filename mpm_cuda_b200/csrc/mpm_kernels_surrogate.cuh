@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
                     source_from_tau<D>(v, Cn, tau, g, sc.dt_next, src);
                     ++n_net;
                 } else {
-                    particle_stress_source<D, MAT>(v, Cn, F, 1.f, g, sc.dt_next, src);
+                    particle_stress_source<D, MAT, true>(v, Cn, F, 1.f, g, sc.dt_next, src);
                     ++n_svd;
                 }
                 scatter_global<D, PAGED>(sn, src, sc, o, A, tb, wpages);

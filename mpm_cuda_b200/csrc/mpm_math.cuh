@@ -292,7 +292,7 @@ MPM_HD void svd(const float* F, float* U, float* s, float* V) {
 // smallest one is negated (the convention of the SVD: s0 >= s1 >= |s2|, the
 // last carrying the sign of det F).  The sum over k does not depend on the
 // order of the eigenpairs, so they are not sorted.
-MPM_HD void kirchhoff_fcr3_eig(const float* F, float mu, float lambda, float* tau) {
+MPM_HD void kirchhoff_fcr3(const float* F, float mu, float lambda, float* tau) {
     float S[9], U[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -329,6 +329,30 @@ MPM_HD void kirchhoff_fcr3_eig(const float* F, float mu, float lambda, float* ta
         }
 }
 
+template <int D>
+MPM_HD void kirchhoff_fcr(const float* F, float mu, float lambda, float* tau) {
+    if constexpr (D == 3) {
+        kirchhoff_fcr3(F, mu, lambda, tau);
+    } else {
+        float U[4], s[2], V[4];
+        svd2(F, U, s, V);
+        const float J = det<2>(F);
+        const float iso = lambda * J * (J - 1.f);
+        float dg[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) dg[k] = 2.f * mu * s[k] * (s[k] - 1.f);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float acc = (i == j) ? iso : 0.f;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) acc = fmaf(U[i * 2 + k] * dg[k], U[j * 2 + k], acc);
+                tau[i * 2 + j] = acc;
+            }
+    }
+}
+
 // The same stress from the rotation R of F = R S itself, for F that is neither
 // inverted nor near singular:  tau = 2 mu (F - R) F^T + lambda J (J - 1) I.
 // R by Newton's iteration R <- (R + R^-T) / 2 from R = F (Higham, Computing the
@@ -336,11 +360,12 @@ MPM_HD void kirchhoff_fcr3_eig(const float* F, float mu, float lambda, float* ta
 // from above after the first step, so det R - 1 bounds their distance from 1;
 // a step from within 2e-4 leaves 2e-8.  A near-rotation F takes two or three
 // steps of about 45 operations where the eigendecomposition takes two or three
-// sweeps of about 140.
-MPM_HD void kirchhoff_fcr3(const float* F, float mu, float lambda, float* tau) {
+// sweeps of about 140.  The atomic path's passes use it; the deterministic path
+// keeps the eigendecomposition, whose results stay the same from build to build.
+MPM_HD void kirchhoff_polar3(const float* F, float mu, float lambda, float* tau) {
     const float J = det<3>(F);
         if (!(J > 0.02f && J < 50.f)) {
-        kirchhoff_fcr3_eig(F, mu, lambda, tau);
+        kirchhoff_fcr3(F, mu, lambda, tau);
         return;
     }
     float R[9];
@@ -378,30 +403,6 @@ MPM_HD void kirchhoff_fcr3(const float* F, float mu, float lambda, float* tau) {
             tau[i * 3 + j] = acc;
             tau[j * 3 + i] = acc;
         }
-}
-
-template <int D>
-MPM_HD void kirchhoff_fcr(const float* F, float mu, float lambda, float* tau) {
-    if constexpr (D == 3) {
-        kirchhoff_fcr3(F, mu, lambda, tau);
-    } else {
-        float U[4], s[2], V[4];
-        svd2(F, U, s, V);
-        const float J = det<2>(F);
-        const float iso = lambda * J * (J - 1.f);
-        float dg[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) dg[k] = 2.f * mu * s[k] * (s[k] - 1.f);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                float acc = (i == j) ? iso : 0.f;
-#pragma unroll
-                for (int k = 0; k < 2; ++k) acc = fmaf(U[i * 2 + k] * dg[k], U[j * 2 + k], acc);
-                tau[i * 2 + j] = acc;
-            }
-    }
 }
 
 // ------------------------------------------------------------- B-spline --

@@ -84,7 +84,8 @@ __device__ __forceinline__ bool is_mat(const GroupParams& g, int m) {
     return MAT >= 0 ? MAT == m : g.type == m;
 }
 
-template <int D, int MAT = -1>
+// POLAR: the 3D solid stress from the polar iteration (kirchhoff_polar3).
+template <int D, int MAT = -1, bool POLAR = false>
 __device__ __forceinline__ void particle_stress_source(const float* v, const float* C, const float* F,
                                                        float aux, const GroupParams& g, float dt,
                                                        P2GSource<D>& src) {
@@ -103,7 +104,8 @@ __device__ __forceinline__ void particle_stress_source(const float* v, const flo
             mu *= hc;
             la *= hc;
         }
-        kirchhoff_fcr<D>(F, mu, la, tau);
+        if constexpr (POLAR && D == 3) kirchhoff_polar3(F, mu, la, tau);
+        else kirchhoff_fcr<D>(F, mu, la, tau);
     }
     const float k = -dt * g.p_vol;
 #pragma unroll
@@ -117,11 +119,11 @@ __device__ __forceinline__ void particle_stress_source(const float* v, const flo
 }
 
 // the same with the scene's current substep
-template <int D, int MAT = -1>
+template <int D, int MAT = -1, bool POLAR = false>
 __device__ __forceinline__ void particle_stress_source(const float* v, const float* C, const float* F,
                                                        float aux, const GroupParams& g, const SceneParams& sc,
                                                        P2GSource<D>& src) {
-    particle_stress_source<D, MAT>(v, C, F, aux, g, sc.dt, src);
+    particle_stress_source<D, MAT, POLAR>(v, C, F, aux, g, sc.dt, src);
 }
 
 // Left singular vectors and clamped singular values of snow's new elastic F
