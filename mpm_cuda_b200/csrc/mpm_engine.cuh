@@ -185,7 +185,6 @@ struct Engine {
     int prologue();
     int build_graph(int parity, int rebin, int count, cudaGraphExec_t* out);
     void drop_graphs();
-    int unpermute_to_alt();
     bool fused() const { return opt.p2g_mode == MPM_P2G_ATOMIC; }
     bool deterministic() const { return opt.p2g_mode == MPM_P2G_DETERMINISTIC; }
     bool direct() const { return opt.p2g_mode == MPM_P2G_DIRECT; }
