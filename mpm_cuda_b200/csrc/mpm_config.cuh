@@ -78,6 +78,14 @@ constexpr int kNumFusedCfgs = FusedCfgTable::N;
 // fewest particles a chunk of any configuration holds (sizes the chunk lists)
 constexpr int kMinChunkParticles = 64;
 
+// Whether a configuration sums runs: those declared so, which address a dense
+// grid; and in a paged grid the cell-major ones of 128 threads with registers
+// to spare (at most 5 CTAs per SM), which declare the direct scatter
+constexpr bool sums_runs(int cfg, bool paged) {
+    const FusedCfg& c = kFusedCfgs[cfg];
+    return paged ? c.scatter == SCATTER_DIRECT && c.order == ORDER_CELL && c.chunk == 128 && c.min_ctas <= 5
+                 : c.scatter == SCATTER_RUNS;
+}
 // particles per thread of a run-sum chunk at most
 constexpr int kMaxRunRounds = 3;
 // SCATTER_RUNS: float4s of a particle's source record, and the dynamic shared
@@ -85,14 +93,15 @@ constexpr int kMaxRunRounds = 3;
 constexpr int run_rec4(int dim) { return dim == 3 ? 6 : 4; }
 constexpr int run_smem(int dim, int particles) { return particles * (run_rec4(dim) * 16 + 2); }
 // dynamic shared memory of a launch configuration
-constexpr int fused_dyn_smem(int dim, int cfg) {
-    return kFusedCfgs[cfg].scatter == SCATTER_RUNS ? run_smem(dim, kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds) : 0;
+constexpr int fused_dyn_smem(int dim, int cfg, bool paged) {
+    return sums_runs(cfg, paged) ? run_smem(dim, kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds) : 0;
 }
 // the most any configuration of the same instantiation asks for
-constexpr int fused_dyn_smem_max(int dim, int cfg) {
+constexpr int fused_dyn_smem_max(int dim, int cfg, bool paged) {
     int most = 0;
     for (int i = 0; i < kNumFusedCfgs; ++i)
-        if (kFusedCfgs[i].kernel == kFusedCfgs[cfg].kernel && fused_dyn_smem(dim, i) > most) most = fused_dyn_smem(dim, i);
+        if (kFusedCfgs[i].kernel == kFusedCfgs[cfg].kernel && fused_dyn_smem(dim, i, paged) > most)
+            most = fused_dyn_smem(dim, i, paged);
     return most;
 }
 
@@ -104,7 +113,7 @@ constexpr bool fused_cfgs_consistent() {
         if (k.chunk != c.chunk || k.min_ctas != c.min_ctas || k.scatter != c.scatter ||
             (c.order != ORDER_RANK && c.order != ORDER_CELL) ||
             (c.scatter == SCATTER_RUNS && c.order != ORDER_CELL) ||
-            (c.scatter == SCATTER_RUNS && c.rounds > kMaxRunRounds) || c.chunk * c.rounds < kMinChunkParticles ||
+            ((sums_runs(i, false) || sums_runs(i, true)) && c.rounds > kMaxRunRounds) || c.chunk * c.rounds < kMinChunkParticles ||
             c.chunk % 32 != 0)
             return false;
     }

@@ -524,7 +524,7 @@ int Engine::chunk_particles() const { return kFusedCfgs[cfg].chunk * kFusedCfgs[
 
 void Engine::set_config(int ci) {
     cfg = ci;
-    const int dyn = fused_dyn_smem(dim, ci);
+    const int dyn = fused_dyn_smem(dim, ci, paged);
     for (int mat = 0; mat < kMats; ++mat) {
         int per_sm = 0;
         const FusedFn fn = fused_fn(dim, mat, ci, fixed_scene, paged);
@@ -537,7 +537,7 @@ void Engine::set_config(int ci) {
         // function's, shared by every handle: always the most any of its
         // configurations needs
         if (dyn > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            fused_dyn_smem_max(dim, ci)) != cudaSuccess)
+                                            fused_dyn_smem_max(dim, ci, paged)) != cudaSuccess)
             cudaGetLastError();
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kFusedCfgs[ci].chunk, dyn) != cudaSuccess) {
             cudaGetLastError();  // the query failed: fall back to one CTA per SM
@@ -1007,7 +1007,7 @@ void Engine::enqueue_g2p2g(int parity) {
         } else {
             cudaLaunchAttribute attr;
             const cudaLaunchConfig_t lc = pdl_config(fused_ctas[mat], kFusedCfgs[cfg].chunk,
-                                                     fused_dyn_smem(dim, cfg), stream, &attr);
+                                                     fused_dyn_smem(dim, cfg, paged), stream, &attr);
             const cudaError_t e = cudaLaunchKernelEx(&lc, fused_fn(dim, mat, cfg, fixed_scene, paged), buf(parity), A);
             note_launch_status("k_g2p2g", e);
             note_launch("fused_fn");

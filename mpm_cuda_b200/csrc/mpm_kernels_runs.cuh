@@ -181,13 +181,14 @@ __device__ __forceinline__ void sum_plane2(const float4* __restrict__ recs, int 
     } while (slot >= 0);
 }
 
-template <int D, int MAT, int CHUNK, int MINB, bool FIXED>
+template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
     using P = Planes<D>;
     using TS = TileShape<D>;
     using RS = RunShape<D>;
-    constexpr bool TMA = FIXED;
+    constexpr bool TMA = FIXED && !PAGED;
     __shared__ __align__(128) float4 tv[TS::VN];  // the chunk's velocity window
+    __shared__ int s27[2][27];                    // PAGED: the windows' physical blocks
     __shared__ int head[2][RS::N];                // first record of each base's run, -1: none
     __shared__ int cnt[2][RS::N];                 // its length
     __shared__ int n_runs[2];
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
     const int nch = *A.n_chunks;
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
-    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, false>(A, cur, tv, nullptr, &s_ch[0], &s_bar);
+    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, PAGED>(A, cur, tv, s27[0], &s_ch[0], &s_bar);
     cp_async_commit();
     SpeedFlush speed;
     __syncthreads();  // s_bar and the lists initialised
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
                 Stencil<D> st;
                 if (make_stencil<D>(x, sc, st, err)) {
                     G2PAcc<D> acc;
-                    g2p_window<D, false, FIXED>(st, o, tv, sc, A, acc);
+                    g2p_window<D, PAGED, FIXED && !PAGED>(st, o, tv, sc, A, acc);
                     // loaded after the gather, its register peak
                     const GroupParams g = particle_group<FIXED>(A, pb, i);
                     float F[D * D], Cn[D * D], v[D], aux;
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         }
         __syncthreads();  // (2) records, runs and the next chunk's record complete; the window is free
         const int next_chunk = s_next[b];
-        if (next_chunk < nch) load_window<D, CHUNK, FIXED, false>(A, s_ch[b ^ 1], tv, nullptr, &s_bar);
+        if (next_chunk < nch) load_window<D, CHUNK, FIXED, PAGED>(A, s_ch[b ^ 1], tv, s27[b ^ 1], &s_bar);
         cp_async_commit();
         mark_touched<D>(touched[b], sc, o, A);
         speed.fold(ch.scene, &s_speed, A.speed_max);
@@ -377,14 +378,34 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
             PlaneSums acc;
             if constexpr (D == 3) sum_plane3(recs, slot, ox, acc);
             else sum_plane2(recs, slot, acc);
-            const StencilIndex<D> ix(sc, base);
-            float4* gm = A.grid_mom + sc.node_off;
+            auto value = [&](int n) { return make_float4(acc.xy[n].x, acc.xy[n].y, acc.z[n], acc.m[n]); };
+            if constexpr (PAGED) {
+                // a block the stencil covers has no page: the pool ran out or
+                // the particle moved more than a cell since the last grid update
+                if (ox == 0 && !stencil_paged<D>(sc, A.pages, base)) atomicOr(A.err_word, ERR_POOL);
+                if (e & kRunOutside) {
 #pragma unroll
-            for (int n = 0; n < 9; ++n) {
-                int at;
-                if constexpr (D == 3) at = (ox == 0 ? ix.x[0] : ox == 1 ? ix.x[1] : ix.x[2]) + ix.y[n / 3] + ix.z[n % 3];
-                else at = ix(n / 3, n % 3, 0);
-                atomicAdd(&gm[at], make_float4(acc.xy[n].x, acc.xy[n].y, acc.z[n], acc.m[n]));
+                    for (int n = 0; n < 9; ++n)
+                        atomicAdd(&A.grid_mom[grid_node<D, true>(sc, A.pages, base[0] + (D == 3 ? ox : n / 3),
+                                                                 base[1] + (D == 3 ? n / 3 : n % 3),
+                                                                 D == 3 ? base[2] + n % 3 : 0)],
+                                  value(n));
+                } else {
+                    const PagedStencilIndex<D> ix(base, o);
+                    const int x = ox == 0 ? ix.x[0] : ox == 1 ? ix.x[1] : ix.x[2];
+#pragma unroll
+                    for (int n = 0; n < 9; ++n) {
+                        const int p = D == 3 ? x + ix.y[n / 3] + ix.z[n % 3] : ix.x[n / 3] + ix.y[n % 3];
+                        atomicAdd(&A.grid_mom[(long long)s27[b][p & 255] * 64 + (p >> 8)], value(n));
+                    }
+                }
+            } else {
+                const StencilIndex<D> ix(sc, base);
+                float4* gm = A.grid_mom + sc.node_off;
+                const int x = ox == 0 ? ix.x[0] : ox == 1 ? ix.x[1] : ix.x[2];
+#pragma unroll
+                for (int n = 0; n < 9; ++n)
+                    atomicAdd(&gm[D == 3 ? x + ix.y[n / 3] + ix.z[n % 3] : ix(n / 3, n % 3, 0)], value(n));
             }
         }
         cur = next_chunk;

@@ -62,3 +62,26 @@ def test_particles_outside_the_window_are_runs_of_their_own(gpu, d, name):
             sim.step(12)
             compare(sim.get_state(0), orc.state(), {"x": 2e-5, "v": 2e-3, "C": 5e-3, "F": 1e-4, "aux": 1e-4})
             assert sim.bin_stats()[0] > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [33, 257])
+def test_paged_grid(gpu, n):
+    """The cell-major 128-thread configurations of a paged grid sum runs: one long run, and particles that leave their
+    window (tolerances of the two tests above)."""
+    sc = one_cell_scene(3, n, 3 + n)
+    h, dt = sc.h, 1e-4
+    x, v, C, F, aux = S.perturbed_blob(3, S.jello(), n_grid=32, h=h, ppc=2, radius_cells=5.0, seed=92, center=np.full(3, 0.5))
+    v[:] = np.array([1.2, -0.8, 0.6]) * (0.4 * h / dt / 1.2)
+    fast = Scene(dim=3, n=(32,) * 3, h=h, dt=dt, bc_type=L.BC_SLIP, bc_lo=3, bc_hi=3,
+                 groups=[group_from_arrays(S.jello(), h, 2, x, v, 0 * C, F, aux)])
+    orc, orc_fast = oracle_for(sc), oracle_for(fast)
+    assert orc.step(2) == 0 and orc_fast.step(12) == 0
+    for k in (12, 13, 20):
+        with Simulation([sc], kernel_config=k, grid_pool_blocks=512) as sim:
+            sim.step(2)
+            compare(sim.get_state(0), orc.state(), {"x": 2e-6, "v": 1e-4, "C": 5e-3, "F": 1e-5, "aux": 1e-5})
+        with Simulation([fast], kernel_config=k, grid_pool_blocks=512, rebin_interval=32) as sim:
+            sim.step(12)
+            compare(sim.get_state(0), orc_fast.state(), {"x": 2e-5, "v": 2e-3, "C": 5e-3, "F": 1e-4, "aux": 1e-4})
+            assert sim.bin_stats()[0] > 0
