@@ -555,20 +555,21 @@ void Engine::set_config(int ci) {
 // CTAs measured slower), else 64; it takes ceil(chunk_particles() / that)
 // rounds, the last one partly idle when the chunk is not a multiple of it
 int Engine::sur_chunk() const { return chunk_particles() >= 128 ? 128 : 64; }
+int Engine::sur_rounds() const { return (chunk_particles() + sur_chunk() - 1) / sur_chunk(); }
 
 void Engine::sur_occupancy() {
     for (int mat = 0; mat < kMats; ++mat) {
         if (!sur_kernel(mat)) continue;
         const int ch = sur_chunk();
         int per_sm = 0;
-        // the network rows live in dynamic shared memory; with the windows and
-        // weights they can exceed the 48 KB a kernel gets without opting in
+        // the records and network rows live in dynamic shared memory; with the
+        // window and weights they exceed the 48 KB a kernel gets without opting
+        // in (the limit is the function's: always the largest chunk's)
         if (cudaFuncSetAttribute(sur_fn(ch, fixed_scene, paged), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 sur_dyn_smem(ch)) !=
-            cudaSuccess)
+                                 sur_dyn_smem(ch, ch == 64 ? 1 : kSurMaxRounds)) != cudaSuccess)
             cudaGetLastError();  // not fatal here: the occupancy query and the launch report it
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sur_fn(ch, fixed_scene, paged), ch, sur_dyn_smem(ch)) !=
-            cudaSuccess) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sur_fn(ch, fixed_scene, paged), ch,
+                                                          sur_dyn_smem(ch, sur_rounds())) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 1;
         }
@@ -999,9 +1000,9 @@ void Engine::enqueue_g2p2g(int parity) {
             const SurArgs SA{&sur->weights->f, sur->meta, sur_counts};
             const int ch = sur_chunk();
             FusedArgs As = A;
-            As.rounds = (chunk_particles() + ch - 1) / ch;
+            As.rounds = sur_rounds();
             cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t lc = pdl_config(sur_ctas[mat], ch, sur_dyn_smem(ch), stream, &attr);
+            const cudaLaunchConfig_t lc = pdl_config(sur_ctas[mat], ch, sur_dyn_smem(ch, As.rounds), stream, &attr);
             const cudaError_t e = cudaLaunchKernelEx(&lc, sur_fn(ch, fixed_scene, paged), buf(parity), As, SA);
             note_launch_status("k_g2p2g_sur", e);
         } else {

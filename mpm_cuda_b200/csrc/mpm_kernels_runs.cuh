@@ -181,39 +181,68 @@ __device__ __forceinline__ void sum_plane2(const float4* __restrict__ recs, int 
     } while (slot >= 0);
 }
 
-template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
-__global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
+// Shared memory of a run-sum pass
+template <int D>
+struct __align__(128) RunShared {
+    float4 tv[TileShape<D>::VN];      // the chunk's velocity window
+    int hist[kRunBins];               // runs per length, longest first
+    Chunk ch[2];                      // records of this and the next chunk
+    int head[2][RunShape<D>::N];      // first record of each base's run, -1: none
+    int cnt[RunShape<D>::N];          // its length, reset by its reader
+    int s27[2][27];                   // PAGED: the windows' physical blocks
+    int n_runs[2];
+    unsigned touched[2];              // 3^D neighbour-block bits
+    int next[2];
+    unsigned speed;                   // adaptive dt: this chunk's max signal speed
+    unsigned long long bar;
+};
+
+// Puts particle li's P2G source on the list of its base node (phase A)
+template <int D>
+__device__ __forceinline__ void insert_record(RunShared<D>& sm, float4* recs, unsigned short* runs, int b, int li,
+                                              const Stencil<D>& sn, const P2GSource<D>& src, const SceneParams& sc,
+                                              const int* o, const FusedArgs& A) {
+    using RS = RunShape<D>;
+    int next = -1;
+    if (in_window<D>(sn.base, o)) {
+        const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
+        const int key = l0 + RS::B * (l1 + RS::B * l2);
+        next = atomicExch(&sm.head[b][key], li);
+        atomicAdd(&sm.cnt[key], 1);
+        if (next < 0) {
+            runs[atomicAdd(&sm.n_runs[b], 1)] = (unsigned short)key;
+            atomicOr(&sm.touched[b], touched_bits<D>(l0, l1, l2));
+        }
+    } else {
+        atomicAdd(A.fallback, 1u);
+        runs[atomicAdd(&sm.n_runs[b], 1)] = (unsigned short)(kRunOutside | (unsigned)li);
+    }
+    write_record<D>(recs + li * run_rec4(D), sn, src, sc.h, sc.inv_h, next);
+}
+
+// The pass of a CTA over its chunks.  round(ch, sc, o, b, li, speed_bits) is
+// phase A of one particle of every thread (li >= ch.count: none); it puts the
+// P2G source it computes on the lists of parity b with insert_record.  A chunk
+// holds at most CHUNK x MAXR particles.
+template <int D, int CHUNK, int MAXR, bool FIXED, bool PAGED, class Round>
+__device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArgs& A, RunShared<D>& sm, float4* recs,
+                                           unsigned short* runs, Round round) {
     using P = Planes<D>;
-    using TS = TileShape<D>;
     using RS = RunShape<D>;
     constexpr bool TMA = FIXED && !PAGED;
-    __shared__ __align__(128) float4 tv[TS::VN];  // the chunk's velocity window
-    __shared__ int s27[2][27];                    // PAGED: the windows' physical blocks
-    __shared__ int head[2][RS::N];                // first record of each base's run, -1: none
-    __shared__ int cnt[2][RS::N];                 // its length
-    __shared__ int n_runs[2];
-    __shared__ __align__(16) int hist[kRunBins];  // runs per length, longest first
-    __shared__ unsigned touched[2];               // 3^D neighbour-block bits
-    __shared__ int s_next[2];
-    __shared__ __align__(16) Chunk s_ch[2];
-    __shared__ __align__(8) unsigned long long s_bar;
-    __shared__ unsigned s_speed;                  // adaptive dt: this chunk's max signal speed
-    extern __shared__ __align__(16) float4 recs[];
-    unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
-
-    for (int t = threadIdx.x; t < 2 * RS::N; t += CHUNK) {
-        (&head[0][0])[t] = -1;
-        (&cnt[0][0])[t] = 0;
+    for (int t = threadIdx.x; t < RS::N; t += CHUNK) {
+        sm.head[0][t] = sm.head[1][t] = -1;
+        sm.cnt[t] = 0;
     }
-    if (threadIdx.x < kRunBins) hist[threadIdx.x] = 0;
+    if (threadIdx.x < kRunBins) sm.hist[threadIdx.x] = 0;
     if (threadIdx.x < 2) {
-        n_runs[threadIdx.x] = 0;
-        touched[threadIdx.x] = 0u;
+        sm.n_runs[threadIdx.x] = 0;
+        sm.touched[threadIdx.x] = 0u;
     }
     if (threadIdx.x == 0) {
-        s_speed = 0u;
+        sm.speed = 0u;
         if constexpr (TMA) {
-            mbar_init(&s_bar);
+            mbar_init(&sm.bar);
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
     }
@@ -223,10 +252,10 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
     const int nch = *A.n_chunks;
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
-    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, PAGED>(A, cur, tv, s27[0], &s_ch[0], &s_bar);
+    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, PAGED>(A, cur, sm.tv, sm.s27[0], &sm.ch[0], &sm.bar);
     cp_async_commit();
     SpeedFlush speed;
-    __syncthreads();  // s_bar and the lists initialised
+    __syncthreads();  // the barrier and the lists initialised
     for (int k = 0; cur < nch; ++k) {
         const int b = k & 1;
         int nxt = 0;
@@ -234,7 +263,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         cp_async_wait<0>();
         // (1) the window and the chunk's record are there; the last chunk's runs are summed
         if constexpr (TMA) {
-            const bool ok = mbar_wait(&s_bar, (unsigned)k & 1u);
+            const bool ok = mbar_wait(&sm.bar, (unsigned)k & 1u);
             if (__syncthreads_or(!ok)) {  // a window that never arrived: report it and stop
                 if (threadIdx.x == 0) atomicOr(A.err_word, ERR_TIMEOUT);
                 break;
@@ -242,112 +271,70 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         } else {
             __syncthreads();
         }
-        const Chunk ch = s_ch[b];
+        const Chunk ch = sm.ch[b];
         const SceneParams& sc = chunk_scene<FIXED>(A, ch.scene);
         const int o[3] = {ch.o[0], ch.o[1], ch.o[2]};
         unsigned speed_bits = 0u;
 #pragma unroll 1
         for (int r = 0; r < A.rounds; ++r) {
-            const int li = (int)threadIdx.x + r * CHUNK;  // this round's particle of the chunk
-            if (li < ch.count) {
-                const long long i = (long long)ch.start + li;
-                float* S = pb.s;
-                const long long cap = pb.cap;
-                unsigned err = 0;
-                float x[D];
-#pragma unroll
-                for (int a = 0; a < D; ++a) x[a] = S[(P::X + a) * cap + i];
-                Stencil<D> st;
-                if (make_stencil<D>(x, sc, st, err)) {
-                    G2PAcc<D> acc;
-                    g2p_window<D, PAGED, FIXED && !PAGED>(st, o, tv, sc, A, acc);
-                    // loaded after the gather, its register peak
-                    const GroupParams g = particle_group<FIXED>(A, pb, i);
-                    float F[D * D], Cn[D * D], v[D], aux;
-                    ElasticSVD<D> esvd;
-                    err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux,
-                                                    MAT == SNOW ? &esvd : nullptr, A.defer_vc != 0);
-                    if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
-                    Stencil<D> sn;
-                    if (make_stencil<D>(x, sc, sn, err)) {
-                        P2GSource<D> src;
-                        if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
-                        else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
-                        int next = -1;
-                        if (in_window<D>(sn.base, o)) {
-                            const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
-                            const int key = l0 + RS::B * (l1 + RS::B * l2);
-                            next = atomicExch(&head[b][key], li);
-                            atomicAdd(&cnt[b][key], 1);
-                            if (next < 0) {
-                                runs[atomicAdd(&n_runs[b], 1)] = (unsigned short)key;
-                                atomicOr(&touched[b], touched_bits<D>(l0, l1, l2));
-                            }
-                        } else {
-                            atomicAdd(A.fallback, 1u);
-                            runs[atomicAdd(&n_runs[b], 1)] = (unsigned short)(kRunOutside | (unsigned)li);
-                        }
-                        write_record<D>(recs + li * run_rec4(D), sn, src, sc.h, sc.inv_h, next);
-                    }
-                }
-                if (err) atomicOr(A.err_word, err);
-            }
+            round(ch, sc, o, b, (int)threadIdx.x + r * CHUNK, speed_bits);
             // the next chunk's record, on its way while the rest of this phase runs
             if (r == 0 && threadIdx.x == 0 && nxt < nch) {
                 const char* from = reinterpret_cast<const char*>(&A.chunks[nxt]);
-                char* to = reinterpret_cast<char*>(&s_ch[b ^ 1]);
+                char* to = reinterpret_cast<char*>(&sm.ch[b ^ 1]);
                 cp_async16(to, from, true);
                 cp_async16(to + 16, from + 16, true);
             }
         }
-        if (A.speed_max) speed_warp_reduce(speed_bits, &s_speed);
+        if (A.speed_max) speed_warp_reduce(speed_bits, &sm.speed);
         if (threadIdx.x == 0) {
-            s_next[b] = nxt;
+            sm.next[b] = nxt;
             cp_async_commit();
             cp_async_wait<0>();
         }
         __syncthreads();  // (2) records, runs and the next chunk's record complete; the window is free
-        const int next_chunk = s_next[b];
-        if (next_chunk < nch) load_window<D, CHUNK, FIXED, PAGED>(A, s_ch[b ^ 1], tv, s27[b ^ 1], &s_bar);
+        const int next_chunk = sm.next[b];
+        if (next_chunk < nch) load_window<D, CHUNK, FIXED, PAGED>(A, sm.ch[b ^ 1], sm.tv, sm.s27[b ^ 1], &sm.bar);
         cp_async_commit();
-        mark_touched<D>(touched[b], sc, o, A);
-        speed.fold(ch.scene, &s_speed, A.speed_max);
+        mark_touched<D>(sm.touched[b], sc, o, A);
+        speed.fold(ch.scene, &sm.speed, A.speed_max);
         // the other parity's lists were last read before barrier (1)
-        for (int t = threadIdx.x; t < RS::N; t += CHUNK) {
-            head[b ^ 1][t] = -1;
-            cnt[b ^ 1][t] = 0;
-        }
+        for (int t = threadIdx.x; t < RS::N; t += CHUNK) sm.head[b ^ 1][t] = -1;
         if (threadIdx.x == 0) {
-            n_runs[b ^ 1] = 0;
-            touched[b ^ 1] = 0u;
+            sm.n_runs[b ^ 1] = 0;
+            sm.touched[b ^ 1] = 0u;
         }
         // the runs by length, the longest first, so that the lanes of a warp
         // walk runs of about one length: a run's place is the number of longer
         // runs plus its rank among those of its length
-        const int nr = n_runs[b];
-        unsigned entry[kMaxRunRounds];
-        int bin[kMaxRunRounds], rank[kMaxRunRounds];
+        const int nr = sm.n_runs[b];
+        unsigned entry[MAXR];
+        int bin[MAXR], rank[MAXR];
 #pragma unroll
-        for (int q = 0; q < kMaxRunRounds; ++q) {
+        for (int q = 0; q < MAXR; ++q) {
             const int t = (int)threadIdx.x + q * CHUNK;
             if (t < nr) {
                 entry[q] = runs[t];
-                const int len = (entry[q] & kRunOutside) ? 1 : cnt[b][entry[q]];
+                int len = 1;
+                if (!(entry[q] & kRunOutside)) {
+                    len = sm.cnt[entry[q]];
+                    sm.cnt[entry[q]] = 0;
+                }
                 bin[q] = kRunBins - min(len, kRunBins);
-                rank[q] = atomicAdd(&hist[bin[q]], 1);
+                rank[q] = atomicAdd(&sm.hist[bin[q]], 1);
             }
         }
         __syncthreads();  // (3)
 #pragma unroll
-        for (int q = 0; q < kMaxRunRounds; ++q) {
+        for (int q = 0; q < MAXR; ++q) {
             if ((int)threadIdx.x + q * CHUNK < nr) {
                 int at = rank[q];
-                for (int j = 0; j < bin[q]; ++j) at += hist[j];
+                for (int j = 0; j < bin[q]; ++j) at += sm.hist[j];
                 runs[at] = (unsigned short)entry[q];
             }
         }
         __syncthreads();  // (4)
-        if (threadIdx.x < kRunBins) hist[threadIdx.x] = 0;
+        if (threadIdx.x < kRunBins) sm.hist[threadIdx.x] = 0;
         // ---- phase B
         const int items = nr * RS::PLANES;
         for (int it = threadIdx.x; it < items; it += CHUNK) {
@@ -369,7 +356,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
                 for (int a = 0; a < D; ++a) base[a] = sn.base[a];
                 if (ox == 0) mark_stencil<D>(base, sc, A.blk_flag, A.active, A.n_active);
             } else {
-                slot = head[b][e];
+                slot = sm.head[b][e];
                 const int l12 = (int)e / RS::B;
                 base[0] += (int)e - RS::B * l12;
                 base[1] += D == 3 ? l12 % RS::B : l12;
@@ -396,7 +383,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
 #pragma unroll
                     for (int n = 0; n < 9; ++n) {
                         const int p = D == 3 ? x + ix.y[n / 3] + ix.z[n % 3] : ix.x[n / 3] + ix.y[n % 3];
-                        atomicAdd(&A.grid_mom[(long long)s27[b][p & 255] * 64 + (p >> 8)], value(n));
+                        atomicAdd(&A.grid_mom[(long long)sm.s27[b][p & 255] * 64 + (p >> 8)], value(n));
                     }
                 }
             } else {
@@ -411,6 +398,46 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         cur = next_chunk;
     }
     speed.flush(A.speed_max);
+}
+
+template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
+__global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
+    using P = Planes<D>;
+    __shared__ RunShared<D> sm;
+    extern __shared__ __align__(16) float4 recs[];
+    unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
+    run_chunks<D, CHUNK, kMaxRunRounds, FIXED, PAGED>(pb, A, sm, recs, runs,
+                                                      [&](const Chunk& ch, const SceneParams& sc, const int* o, int b,
+                                                          int li, unsigned& speed_bits) {
+        if (li >= ch.count) return;
+        const long long i = (long long)ch.start + li;
+        float* S = pb.s;
+        const long long cap = pb.cap;
+        unsigned err = 0;
+        float x[D];
+#pragma unroll
+        for (int a = 0; a < D; ++a) x[a] = S[(P::X + a) * cap + i];
+        Stencil<D> st;
+        if (make_stencil<D>(x, sc, st, err)) {
+            G2PAcc<D> acc;
+            g2p_window<D, PAGED, FIXED && !PAGED>(st, o, sm.tv, sc, A, acc);
+            // loaded after the gather, its register peak
+            const GroupParams g = particle_group<FIXED>(A, pb, i);
+            float F[D * D], Cn[D * D], v[D], aux;
+            ElasticSVD<D> esvd;  // snow: the plasticity step's decomposition, reused by the stress
+            err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux, MAT == SNOW ? &esvd : nullptr,
+                                            A.defer_vc != 0);
+            if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
+            Stencil<D> sn;
+            if (make_stencil<D>(x, sc, sn, err)) {
+                P2GSource<D> src;
+                if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
+                else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
+                insert_record<D>(sm, recs, runs, b, li, sn, src, sc, o, A);
+            }
+        }
+        if (err) atomicOr(A.err_word, err);
+    });
 }
 
 }  // namespace mpm

@@ -155,11 +155,19 @@ __device__ __forceinline__ void init_bias(float (*acc)[4], const float* b, int l
 // 16 outputs (columns >= 9 are padding), both with row stride XS floats in
 // shared memory (an odd XS keeps the per-particle row accesses free of bank
 // conflicts); y may alias x.  All 32 lanes of the warp must call it together.
-template <int XS = IN_PAD>
+// BF16_ROWS: the features are already packed to BF16 pairs (8 words a row).
+template <int XS = IN_PAD, bool BF16_ROWS = false>
 __device__ __forceinline__ void forward_tile(const Forward& W, const float* x, float* y, int lane) {
     const int g = lane >> 2, t = lane & 3;
     unsigned a[4];
-    {
+    if constexpr (BF16_ROWS) {
+        const float* r0 = x + g * XS;
+        const float* r1 = x + (g + 8) * XS;
+        a[0] = __float_as_uint(r0[t]);
+        a[1] = __float_as_uint(r1[t]);
+        a[2] = __float_as_uint(r0[t + 4]);
+        a[3] = __float_as_uint(r1[t + 4]);
+    } else {
         const float* r0 = x + g * XS;
         const float* r1 = x + (g + 8) * XS;
         a[0] = pack_bf16(r0[2 * t], r0[2 * t + 1]);
