@@ -695,7 +695,7 @@ template <int D, int MAT>
 __device__ __forceinline__ unsigned update_and_store(const G2PAcc<D>& acc, const SceneParams& sc, const GroupParams& g,
                                                      float* __restrict__ S, long long cap, long long i, float* x,
                                                      float* v, float* Cn, float* F, float& aux,
-                                                     ElasticSVD<D>* keep = nullptr, bool defer_vc = false) {
+                                                     typename SnowKeep<D>::T* keep = nullptr, bool defer_vc = false) {
     using P = Planes<D>;
     aux = 1.f;
     if (MAT != JELLO) aux = S[P::AUX * cap + i];
@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
                     // loaded after the gather, its register peak
                     const GroupParams g = particle_group<FIXED>(A, pb, i);
                     float F[D * D], Cn[D * D], v[D], aux;
-                    ElasticSVD<D> esvd;  // snow: the plasticity step's decomposition, reused by the stress
+                    typename SnowKeep<D>::T esvd;  // snow: the plasticity step's decomposition, reused by the stress
                     err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux,
                                                     MAT == SNOW ? &esvd : nullptr, A.defer_vc != 0);
                     if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
                     Stencil<D> sn;
                     if (make_stencil<D>(x, sc, sn, err)) {
                         P2GSource<D> src;
-                        if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
+                        if (MAT == SNOW) snow_stress_source(v, Cn, F, esvd, aux, g, sc.dt_next, src);
                         else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
                         scatter_global<D, PAGED>(sn, src, sc, o, A, tb, wpages);
                     }

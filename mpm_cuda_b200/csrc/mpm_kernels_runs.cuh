@@ -424,14 +424,14 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
             // loaded after the gather, its register peak
             const GroupParams g = particle_group<FIXED>(A, pb, i);
             float F[D * D], Cn[D * D], v[D], aux;
-            ElasticSVD<D> esvd;  // snow: the plasticity step's decomposition, reused by the stress
+            typename SnowKeep<D>::T esvd;  // snow: the plasticity step's decomposition, reused by the stress
             err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux, MAT == SNOW ? &esvd : nullptr,
                                             A.defer_vc != 0);
             if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
             Stencil<D> sn;
             if (make_stencil<D>(x, sc, sn, err)) {
                 P2GSource<D> src;
-                if (MAT == SNOW) snow_stress_source<D>(v, Cn, esvd, aux, g, sc.dt_next, src);
+                if (MAT == SNOW) snow_stress_source(v, Cn, F, esvd, aux, g, sc.dt_next, src);
                 else particle_stress_source<D, MAT, true>(v, Cn, F, aux, g, sc.dt_next, src);
                 insert_record<D>(sm, recs, runs, b, li, sn, src, sc, o, A);
             }

@@ -100,8 +100,9 @@ MPM_HD float fast_half_inverse(float x) {
 #endif
 }
 
-// one Jacobi rotation on the (p,q) pair of the symmetric S (stored as 3x3)
-template <int P, int Q>
+// one Jacobi rotation on the (p,q) pair of the symmetric S (stored as 3x3),
+// applied to the columns of V too when VECS
+template <int P, int Q, bool VECS = true>
 MPM_HD void jacobi_rotate(float* S, float* V) {
     constexpr int R = 3 - P - Q;  // the remaining index
     const float spq = S[P * 3 + Q];
@@ -126,11 +127,13 @@ MPM_HD void jacobi_rotate(float* S, float* V) {
     const float nrp = c * srp - s * srq, nrq = s * srp + c * srq;
     S[R * 3 + P] = nrp; S[P * 3 + R] = nrp;
     S[R * 3 + Q] = nrq; S[Q * 3 + R] = nrq;
+    if constexpr (VECS) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float vkp = V[k * 3 + P], vkq = V[k * 3 + Q];
-        V[k * 3 + P] = c * vkp - s * vkq;
-        V[k * 3 + Q] = s * vkp + c * vkq;
+        for (int k = 0; k < 3; ++k) {
+            const float vkp = V[k * 3 + P], vkq = V[k * 3 + Q];
+            V[k * 3 + P] = c * vkp - s * vkq;
+            V[k * 3 + Q] = s * vkp + c * vkq;
+        }
     }
 }
 
@@ -140,6 +143,23 @@ MPM_HD bool jacobi_converged(const float* S) {
     const float off = S[1] * S[1] + S[2] * S[2] + S[5] * S[5];
     const float dg = S[0] * S[0] + S[4] * S[4] + S[8] * S[8];
     return off <= 1e-14f * dg;
+}
+
+// Eigenvalues of the symmetric E (destroyed), descending: up to 4 Jacobi sweeps
+// without vectors, until the off-diagonal mass is below 3e-8, which bounds
+// their error
+MPM_HD void sym_eigenvalues3(float* E, float* e) {
+#pragma unroll 1
+    for (int sweep = 0; sweep < 4; ++sweep) {
+        if (sweep >= 2 && E[1] * E[1] + E[2] * E[2] + E[5] * E[5] <= 1e-15f) break;
+        jacobi_rotate<0, 1, false>(E, nullptr);
+        jacobi_rotate<0, 2, false>(E, nullptr);
+        jacobi_rotate<1, 2, false>(E, nullptr);
+    }
+    const float hi = fmaxf(E[0], E[4]), lo = fminf(E[0], E[4]);
+    e[0] = fmaxf(hi, E[8]);
+    e[1] = fmaxf(lo, fminf(hi, E[8]));
+    e[2] = fminf(lo, E[8]);
 }
 
 MPM_HD void swap_cols_neg(float* V, float* lam, int a, int b) {
@@ -362,13 +382,10 @@ MPM_HD void kirchhoff_fcr(const float* F, float mu, float lambda, float* tau) {
 // steps of about 45 operations where the eigendecomposition takes two or three
 // sweeps of about 140.  The atomic path's passes use it; the deterministic path
 // keeps the eigendecomposition, whose results stay the same from build to build.
-MPM_HD void kirchhoff_polar3(const float* F, float mu, float lambda, float* tau) {
-    const float J = det<3>(F);
-        if (!(J > 0.02f && J < 50.f)) {
-        kirchhoff_fcr3(F, mu, lambda, tau);
-        return;
-    }
-    float R[9];
+
+// the rotation R of F, J = det F; false, and no R, where the iteration is not used
+MPM_HD bool polar3(const float* F, float J, float* R) {
+    if (!(J > 0.02f && J < 50.f)) return false;
 #pragma unroll
     for (int k = 0; k < 9; ++k) R[k] = F[k];
 #pragma unroll 1
@@ -389,10 +406,15 @@ MPM_HD void kirchhoff_polar3(const float* F, float mu, float lambda, float* tau)
         for (int k = 0; k < 9; ++k) R[k] = fmaf(half_inv, K[k], 0.5f * R[k]);
         if (it > 0 && !(d > 1.0002f)) break;
     }
+    return true;
+}
+
+// tau from F, its distance Dr = F - R from its rotation and J = det F
+MPM_HD void kirchhoff_from_strain3(const float* F, const float* Dr, float J, float mu, float lambda, float* tau) {
     const float iso = lambda * J * (J - 1.f);
     float E[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) E[k] = 2.f * mu * (F[k] - R[k]);
+    for (int k = 0; k < 9; ++k) E[k] = 2.f * mu * Dr[k];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -403,6 +425,18 @@ MPM_HD void kirchhoff_polar3(const float* F, float mu, float lambda, float* tau)
             tau[i * 3 + j] = acc;
             tau[j * 3 + i] = acc;
         }
+}
+
+MPM_HD void kirchhoff_polar3(const float* F, float mu, float lambda, float* tau) {
+    const float J = det<3>(F);
+    float R[9];
+    if (!polar3(F, J, R)) {
+        kirchhoff_fcr3(F, mu, lambda, tau);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) R[k] = F[k] - R[k];
+    kirchhoff_from_strain3(F, R, J, mu, lambda, tau);
 }
 
 // ------------------------------------------------------------- B-spline --

@@ -140,7 +140,7 @@ struct ElasticSVD {
 // particle_stress_source of Fe = U diag(s) V^T): hardening exp(xi (1 - Jp))
 // (MPMCUDA.cu:342-347) and the fixed-corotated stress of U, s.
 template <int D>
-__device__ __forceinline__ void snow_stress_source(const float* v, const float* C, const ElasticSVD<D>& e,
+__device__ __forceinline__ void snow_stress_source(const float* v, const float* C, const float*, const ElasticSVD<D>& e,
                                                    float aux, const GroupParams& g, float dt, P2GSource<D>& src) {
     const float hc = expf(g.xi * (1.f - aux));
     const float mu = g.mu * hc, la = g.lambda * hc;
@@ -164,6 +164,143 @@ __device__ __forceinline__ void snow_stress_source(const float* v, const float* 
         }
 #pragma unroll
     for (int a = 0; a < D; ++a) src.mv[a] = g.p_mass * v[a];
+    src.m = g.p_mass;
+}
+
+// The 3D fused passes' snow: the distance Fe - R of the new elastic F from its
+// rotation and its determinant, kept for the stress of the next P2G.
+struct ElasticPolar {
+    float Dr[9];
+    float J;
+};
+template <int D>
+struct SnowKeep {
+    using T = ElasticSVD<D>;
+};
+template <>
+struct SnowKeep<3> {
+    using T = ElasticPolar;
+};
+
+// F and aux = det Fp after the Stomakhin clamp of the trial F (Fn).  Most of
+// the material is elastic in a substep: with R from the polar iteration, the
+// strain E = R^T Fn - I has its eigenvalues inside [-theta_c, theta_s] when
+// E + theta_c I and theta_s I - E are positive definite (leading minors), and
+// then nothing is clamped, Fe = Fn.  Else Fe = Fn + R h(E) with h(e) =
+// clamp(e) - e, a matrix function that needs only the eigenvalues e_k of E:
+// in Newton's form over them,
+//   h(E) = h_0 I + h_01 (E - e_0 I) + h_012 (E - e_0 I)(E - e_1 I),
+// whose divided differences of h, a piecewise linear function with slopes 0 and
+// -1, stay bounded however close the eigenvalues are.  An F outside the polar
+// iteration's range takes the singular value decomposition.  (Decomposing every
+// particle, two to four Jacobi sweeps a warp, took 268 us a substep on the 256^3
+// snow scene; now 231 us in flight and 269 us, against 284, once the balls
+// collide and most warps hold a clamped particle.  Against 64 bits, rms: Fe
+// 1.6e-7 -> 2.8e-8, det Fp 1.7e-7 -> 8.9e-8 at stretches exp(0.01 N).)
+__device__ __forceinline__ void snow_clamp3(const float* Fn, const GroupParams& g, float* F, float& aux,
+                                            ElasticPolar& keep) {
+    const float Jt = det<3>(Fn);
+    float R[9];
+    if (polar3(Fn, Jt, R)) {
+        float E[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            F[k] = Fn[k];
+            keep.Dr[k] = Fn[k] - R[k];
+        }
+        keep.J = Jt;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j)
+                E[i * 3 + j] = E[j * 3 + i] =
+                    R[i] * keep.Dr[j] + R[3 + i] * keep.Dr[3 + j] + R[6 + i] * keep.Dr[6 + j];
+        auto positive = [&](float sign, float c) {  // c I + sign E positive definite
+            const float a = fmaf(sign, E[0], c), d = fmaf(sign, E[4], c), f = fmaf(sign, E[8], c);
+            const float m2 = a * d - E[1] * E[1];
+            const float m3 = f * m2 + 2.f * sign * E[1] * E[2] * E[5] - a * E[5] * E[5] - d * E[2] * E[2];
+            return a > 0.f && m2 > 0.f && m3 > 0.f;
+        };
+        if (positive(1.f, g.theta_c) && positive(-1.f, g.theta_s)) return;
+        float W[9], e[3], h[3];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) W[k] = E[k];
+        sym_eigenvalues3(W, e);
+        float Je = 1.f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float c = fminf(fmaxf(e[k], -g.theta_c), g.theta_s);
+            h[k] = c - e[k];
+            Je *= 1.f + c;
+        }
+        const float d01 = e[0] - e[1], d12 = e[1] - e[2], d02 = e[0] - e[2];
+        const float h01 = d01 > 0.f ? __fdividef(h[0] - h[1], d01) : (h[0] != 0.f ? -1.f : 0.f);
+        const float h12 = d12 > 0.f ? __fdividef(h[1] - h[2], d12) : (h[1] != 0.f ? -1.f : 0.f);
+        const float h012 = d02 > 0.f ? __fdividef(h01 - h12, d02) : 0.f;
+        float H[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j) {
+                float p = 0.f;
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    p = fmaf(E[i * 3 + k] - (i == k ? e[0] : 0.f), E[k * 3 + j] - (k == j ? e[1] : 0.f), p);
+                const float q = E[i * 3 + j] - (i == j ? e[0] : 0.f);
+                H[i * 3 + j] = H[j * 3 + i] = fmaf(h012, p, fmaf(h01, q, i == j ? h[0] : 0.f));
+            }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const float t = R[i * 3] * H[j] + R[i * 3 + 1] * H[3 + j] + R[i * 3 + 2] * H[6 + j];
+                F[i * 3 + j] += t;
+                keep.Dr[i * 3 + j] += t;
+            }
+        // det Fp_new = det(Fe_new^-1 Fe_trial Fp) = det_trial / det_new * det Fp
+        aux = aux * (Jt / Je);
+        keep.J = Je;
+        return;
+    }
+    float U[9], s[3], V[9];
+    svd3(Fn, U, s, V);
+    float Je = 1.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = fminf(fmaxf(s[k], 1.f - g.theta_c), 1.f + g.theta_s);
+        Je *= s[k];
+    }
+    // Fe = U diag(s*) V^T, Fe - R = U diag(s* - 1) V^T
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            float fe = 0.f, d = 0.f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                fe = fmaf(U[i * 3 + k] * s[k], V[j * 3 + k], fe);
+                d = fmaf(U[i * 3 + k] * (s[k] - 1.f), V[j * 3 + k], d);
+            }
+            F[i * 3 + j] = fe;
+            keep.Dr[i * 3 + j] = d;
+        }
+    aux = aux * (Jt / Je);
+    keep.J = Je;
+}
+
+__device__ __forceinline__ void snow_stress_source(const float* v, const float* C, const float* F, const ElasticPolar& e,
+                                                   float aux, const GroupParams& g, float dt, P2GSource<3>& src) {
+    const float hc = expf(g.xi * (1.f - aux));
+    float tau[9];
+    kirchhoff_from_strain3(F, e.Dr, e.J, g.mu * hc, g.lambda * hc, tau);
+    const float k = -dt * g.p_vol;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        src.A[i] = k * tau[i];
+        src.mC[i] = g.p_mass * C[i];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) src.mv[a] = g.p_mass * v[a];
     src.m = g.p_mass;
 }
 
@@ -463,10 +600,11 @@ __device__ __forceinline__ float signal_speed(const float* v, const GroupParams&
 
 // Material update after G2P (MPMCUDA.cu:588-713, MPMSnow.py:135-150,
 // MPMWater.py:138).  Updates F / aux in place, returns error bits.
+// keep: the fused passes' snow, whose stress follows in the same pass.
 template <int D, int MAT = -1>
 __device__ __forceinline__ unsigned material_update(const G2PAcc<D>& acc, float dt,
                                                     const GroupParams& g, float* F, float& aux,
-                                                    ElasticSVD<D>* keep = nullptr) {
+                                                    typename SnowKeep<D>::T* keep = nullptr) {
     unsigned err = 0;
     if (is_mat<MAT>(g, WATER)) {
         float div = 0.f;
@@ -483,6 +621,13 @@ __device__ __forceinline__ unsigned material_update(const G2PAcc<D>& acc, float 
         for (int b = 0; b < D; ++b) L[a * D + b] = (a == b ? 1.f : 0.f) + dt * acc.G[a * D + b];
     float Fn[D * D];
     matmul<D>(L, F, Fn);  // F <- (I + dt grad v) F
+    if constexpr (D == 3 && MAT == SNOW) {
+        if (keep) {
+            snow_clamp3(Fn, g, F, aux, *keep);
+            if (!(aux > 0.f)) err |= ERR_DET;
+            return err;
+        }
+    }
     if (is_mat<MAT>(g, SNOW)) {
         // Stomakhin et al. 2013 clamp of the trial elastic F
         float U[D * D], s[D], V[D * D];
@@ -504,11 +649,13 @@ __device__ __forceinline__ unsigned material_update(const G2PAcc<D>& acc, float 
                 for (int k = 0; k < D; ++k) acc2 = fmaf(U[i * D + k] * s[k], V[j * D + k], acc2);
                 F[i * D + j] = acc2;
             }
-        if (keep) {
+        if constexpr (D == 2) {
+            if (keep) {
 #pragma unroll
-            for (int k = 0; k < D * D; ++k) keep->U[k] = U[k];
+                for (int k = 0; k < D * D; ++k) keep->U[k] = U[k];
 #pragma unroll
-            for (int k = 0; k < D; ++k) keep->s[k] = s[k];
+                for (int k = 0; k < D; ++k) keep->s[k] = s[k];
+            }
         }
         // det Fp_new = det(Fe_new^-1 Fe_trial Fp) = det_trial / det_new * det Fp
         aux = aux * (det_trial / det_new);
