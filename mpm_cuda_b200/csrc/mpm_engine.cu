@@ -986,7 +986,7 @@ void Engine::enqueue_grid_update() {
                                              blk_flag, blk_epoch, (const int*)(counters + CNT_EPOCH),
                                              (const SceneParams*)scenes_d, n_scenes, counters + CNT_CURSOR, (int)kMats,
                                              (unsigned*)(counters + CNT_UPDATE_DONE), scenes_h[0],
-                                             vel_linear_mode() ? 1 : 0, pages, err_d);
+                                             vel_linear_mode() ? 1 : 0, pages, err_d, (int)total_blocks);
     note_launch_status("k_grid_update_active", e);
 }
 
@@ -1025,8 +1025,9 @@ void Engine::enqueue_fused_substep(int parity) {
 void Engine::enqueue_adapt_dt() {
     if (!opt.adaptive_dt) return;
     const int n_scenes = (int)scenes_h.size();
-    k_adapt_dt<<<(n_scenes + 127) / 128, 128, 0, stream>>>(scenes_d, n_scenes, speed_max, scene_time);
-    note_launch("k_adapt_dt");
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t lc = pdl_config((unsigned)((n_scenes + 127) / 128), 128, 0, stream, &attr);
+    note_launch_status("k_adapt_dt", cudaLaunchKernelEx(&lc, k_adapt_dt, scenes_d, n_scenes, speed_max, scene_time));
 }
 
 // deterministic P2G of the current state into grid_mom (blocks marked active)

@@ -417,13 +417,17 @@ __global__ void __launch_bounds__(256) k_grid_update_active(float4* __restrict__
                                                             const SceneParams* __restrict__ scenes, int n_scenes,
                                                             int* __restrict__ cursors, int n_cursors,
                                                             unsigned* __restrict__ done, SceneParams fixed_scene,
-                                                            int vel_linear, GridPages gp, unsigned* __restrict__ err_word) {
+                                                            int vel_linear, GridPages gp, unsigned* __restrict__ err_word,
+                                                            int n_blocks) {
     pdl_wait();
+    const int lane = threadIdx.x & 63;
+    int e = blockIdx.x * 4 + (threadIdx.x >> 6);
+    // the first entry on its way together with the count (the list has an entry
+    // per block: beyond the count a stale one, not used)
+    int b = active[min(e, n_blocks - 1)];
     const int na = *n_active;
     const int ep = *epoch;
-    const int lane = threadIdx.x & 63;
-    for (int e = blockIdx.x * 4 + (threadIdx.x >> 6); e < na; e += gridDim.x * 4) {
-        const int b = active[e];
+    for (; e < na; e += gridDim.x * 4, b = e < na ? active[e] : 0) {
         const SceneParams& sc = FIXED ? fixed_scene : scenes[scene_of_block(scenes, n_scenes, b)];
         int ix, iy, iz;
         block_node_coords<D>(sc, b - sc.block_off, lane, ix, iy, iz);
@@ -1059,6 +1063,10 @@ __global__ void __launch_bounds__(256) k_recover_vc(ParticleBuf pb, long long n,
 // dt_min, dt_max) from the speeds this pass saw.  (The reference computes a
 // max(J, 1/J)^3 factor for this and never applies it, MPMCUDA.cu:915-920.)
 static __global__ void k_adapt_dt(SceneParams* scenes, int n_scenes, unsigned* speed_max, double* scene_time) {
+    // the grid update behind it may launch at once: it waits for this kernel to
+    // end, and this one for the fused pass
+    pdl_trigger();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_scenes) return;
     SceneParams& sc = scenes[s];

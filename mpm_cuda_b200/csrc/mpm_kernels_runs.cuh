@@ -220,8 +220,15 @@ __device__ __forceinline__ void insert_record(RunShared<D>& sm, float4* recs, un
     write_record<D>(recs + li * run_rec4(D), sn, src, sc.h, sc.inv_h, next);
 }
 
-// The pass of a CTA over its chunks.  round(ch, sc, o, b, li, speed_bits) is
-// phase A of one particle of every thread (li >= ch.count: none); it puts the
+template <int D>
+__device__ __forceinline__ void load_position(const ParticleBuf& pb, long long i, float* x) {
+#pragma unroll
+    for (int a = 0; a < D; ++a) x[a] = pb.s[(Planes<D>::X + a) * pb.cap + i];
+}
+
+// The pass of a CTA over its chunks.  round(ch, sc, o, b, li, x, speed_bits) is
+// phase A of one particle of every thread (li >= ch.count: none), at position x
+// (the round may overwrite it); it puts the
 // P2G source it computes on the lists of parity b with insert_record.  A chunk
 // holds at most CHUNK x MAXR particles.
 template <int D, int CHUNK, int MAXR, bool FIXED, bool PAGED, class Round>
@@ -246,20 +253,30 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
     }
-    pdl_wait();     // the grid update ahead of this launch has finished
-    pdl_trigger();  // the next pass may launch; it waits for this one to end
-    if (A.bump_epoch && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.epoch, 1);
+    // The chunk list and the particles were last written before the grid update
+    // ahead of this launch began: a CTA starts once that kernel's CTAs (or those
+    // of another material's pass, which wait for it) have all passed their own
+    // wait.  So the first chunk's record and positions are fetched before this
+    // kernel's wait; velocities, cursors and block flags after it.
     const int nch = *A.n_chunks;
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
-    if (cur < nch) prefetch_velocity_tile<D, CHUNK, FIXED, PAGED>(A, cur, sm.tv, sm.s27[0], &sm.ch[0], &sm.bar);
+    if (threadIdx.x == 0 && cur < nch) sm.ch[0] = A.chunks[cur];
+    __syncthreads();  // the record, the barrier and the lists initialised
+    pdl_wait();     // the grid update ahead of this launch has finished
+    pdl_trigger();  // the next pass may launch; it waits for this one to end
+    if (A.bump_epoch && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.epoch, 1);
+    if (cur < nch) load_window<D, CHUNK, FIXED, PAGED>(A, sm.ch[0], sm.tv, sm.s27[0], &sm.bar);
     cp_async_commit();
     SpeedFlush speed;
-    __syncthreads();  // the barrier and the lists initialised
     for (int k = 0; cur < nch; ++k) {
         const int b = k & 1;
         int nxt = 0;
         if (threadIdx.x == 0) nxt = (int)gridDim.x + atomicAdd(A.cursor, 1);
+        const Chunk ch = sm.ch[b];
+        // the first round's positions, on their way while the window arrives
+        float x[D];
+        if ((int)threadIdx.x < ch.count) load_position<D>(pb, (long long)ch.start + threadIdx.x, x);
         cp_async_wait<0>();
         // (1) the window and the chunk's record are there; the last chunk's runs are summed
         if constexpr (TMA) {
@@ -271,13 +288,14 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
         } else {
             __syncthreads();
         }
-        const Chunk ch = sm.ch[b];
         const SceneParams& sc = chunk_scene<FIXED>(A, ch.scene);
         const int o[3] = {ch.o[0], ch.o[1], ch.o[2]};
         unsigned speed_bits = 0u;
 #pragma unroll 1
         for (int r = 0; r < A.rounds; ++r) {
-            round(ch, sc, o, b, (int)threadIdx.x + r * CHUNK, speed_bits);
+            const int li = (int)threadIdx.x + r * CHUNK;
+            if (r > 0 && li < ch.count) load_position<D>(pb, (long long)ch.start + li, x);
+            round(ch, sc, o, b, li, x, speed_bits);
             // the next chunk's record, on its way while the rest of this phase runs
             if (r == 0 && threadIdx.x == 0 && nxt < nch) {
                 const char* from = reinterpret_cast<const char*>(&A.chunks[nxt]);
@@ -402,21 +420,17 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
 
 template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
-    using P = Planes<D>;
     __shared__ RunShared<D> sm;
     extern __shared__ __align__(16) float4 recs[];
     unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
     run_chunks<D, CHUNK, kMaxRunRounds, FIXED, PAGED>(pb, A, sm, recs, runs,
                                                       [&](const Chunk& ch, const SceneParams& sc, const int* o, int b,
-                                                          int li, unsigned& speed_bits) {
+                                                          int li, float* x, unsigned& speed_bits) {
         if (li >= ch.count) return;
         const long long i = (long long)ch.start + li;
         float* S = pb.s;
         const long long cap = pb.cap;
         unsigned err = 0;
-        float x[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) x[a] = S[(P::X + a) * cap + i];
         Stencil<D> st;
         if (make_stencil<D>(x, sc, st, err)) {
             G2PAcc<D> acc;

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
     // every thread runs every round (the network step is warp-synchronous)
     run_chunks<D, CHUNK, kSurMaxRounds, FIXED, PAGED>(pb, A, sm, recs, runs,
                                                       [&](const Chunk& ch, const SceneParams& sc, const int* o, int b,
-                                                          int li, unsigned& speed_bits) {
+                                                          int li, float* x, unsigned& speed_bits) {
         unsigned err = 0;
         bool next = false;      // the particle scatters into the next substep
         bool eligible = false;  // its group takes the network's stress
@@ -79,9 +79,6 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
             float* S = pb.s;
             const long long cap = pb.cap;
             gi = pb.grp[i];
-            float x[D];
-#pragma unroll
-            for (int a = 0; a < D; ++a) x[a] = S[(Planes<D>::X + a) * cap + i];
             Stencil<D> st;
             if (make_stencil<D>(x, sc, st, err)) {
                 G2PAcc<D> acc;
@@ -123,12 +120,13 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
         __syncwarp();
         if (next) {
             const float4 q0 = stash[0], q1 = stash[1], q2 = stash[2], q3 = stash[3], q4 = stash[4], q5 = stash[5];
-            float x[D] = {q0.x, q0.y, q0.z}, v[D] = {q0.w, q1.x, q1.y};
+            const float xn[D] = {q0.x, q0.y, q0.z};
+            float v[D] = {q0.w, q1.x, q1.y};
             float Cn[9] = {q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
             float F[9] = {q3.w, q4.x, q4.y, q4.z, q4.w, q5.x, q5.y, q5.z, q5.w};
             const GroupParams g = A.groups[gi];
             Stencil<D> sn;
-            make_stencil<D>(x, sc, sn, err);  // the stencil found above
+            make_stencil<D>(xn, sc, sn, err);  // the stencil found above
             float tau[D * D];
             bool use = false;
             if (eligible) {
