@@ -388,6 +388,10 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     // driver without tensor maps leaves the run on the table-reading kernels
     if (fixed_scene && !paged && encode_vel_map() != MPM_OK) fixed_scene = false;
     if ((rc = alloc((void**)&err_d, sizeof(unsigned), "err")) != MPM_OK) return rc;
+    if ((e = cudaMallocHost((void**)&err_h, sizeof(unsigned))) != cudaSuccess) {
+        msg = std::string("mpm_create: cudaMallocHost: ") + cudaGetErrorString(e);
+        return MPM_ERR_NOMEM;
+    }
     for (int p = 0; p < 2; ++p) {
         if ((rc = alloc((void**)&keys[p], cap * sizeof(unsigned long long), "sort keys")) != MPM_OK) return rc;
         if ((rc = alloc((void**)&vals[p], cap * sizeof(unsigned), "sort values")) != MPM_OK) return rc;
@@ -756,6 +760,8 @@ void Engine::release() {
                     sur_counts, speed_max, scene_time,
                     pages.page, pages.slot_block, pages.free_slots};
     for (void* p : ptrs) cudaFree(p);
+    cudaFreeHost(err_h);
+    err_h = nullptr;
     pages = GridPages{};
     groups_d = nullptr;
     scenes_d = nullptr;
@@ -1338,11 +1344,12 @@ int Engine::step(int n) {
 
 // ----------------------------------------------------------- queries --
 
+// (a page-locked word: the copy is queued behind the substeps and one wait
+// serves both)
 int Engine::read_errors(uint32_t* bits) {
-    unsigned v = 0;
-    MPM_CUDA_TRY(cudaMemcpyAsync(&v, err_d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream), "read error word");
+    MPM_CUDA_TRY(cudaMemcpyAsync(err_h, err_d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream), "read error word");
     MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
-    *bits = v;
+    *bits = *err_h;
     return MPM_OK;
 }
 
@@ -1353,11 +1360,10 @@ int Engine::clear_errors() {
 }
 
 int Engine::sync_and_check() {
-    MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
-    if (copy_stream) MPM_CUDA_TRY(cudaStreamSynchronize(copy_stream), "copy stream sync");
     uint32_t bits = 0;
     int rc = read_errors(&bits);
     if (rc != MPM_OK) return rc;
+    if (copy_stream) MPM_CUDA_TRY(cudaStreamSynchronize(copy_stream), "copy stream sync");
     if (bits) {
         char b[256];
         std::snprintf(b, sizeof(b), "device error word 0x%x (1 out of grid, 2 non-finite, 4 det<=0, 16 timeout)", bits);

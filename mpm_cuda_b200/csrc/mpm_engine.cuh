@@ -45,6 +45,7 @@ struct Engine {
     float4* grid_mom = nullptr;  // P2G accumulation (momentum, mass)
     float4* grid_vel = nullptr;  // after the grid update (velocity, mass)
     unsigned* err_d = nullptr;
+    unsigned* err_h = nullptr;  // page-locked copy of the error word
 
     // binning and block activity
     // binning: keys[0] = (home block, material, cell) and vals[0] = rank in
