@@ -3,7 +3,6 @@
 #include "mpm_engine.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
 #include <cub/iterator/counting_input_iterator.cuh>
 
@@ -42,6 +41,7 @@ enum {
     CNT_POOL_FREE = 11,  // paged grid: height of the free stack
     CNT_DET_BLOCKS = 12, // deterministic P2G: length of the ascending list of marked blocks
     CNT_DET_RUNS = 13,   // deterministic P2G: number of runs of records sharing a base node
+    CNT_PLACED = 14,     // re-binning: particles given a segment so far
     CNT_N = 16
 };
 
@@ -452,8 +452,6 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
         sort_tmp_bytes = std::max(sort_tmp_bytes, sel);
     }
     if ((rc = alloc(&sort_tmp, sort_tmp_bytes, "sort temp")) != MPM_OK) return rc;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp_bytes, seg_count, seg_start, (int)(total_blocks * 4));
-    if ((rc = alloc(&scan_tmp, scan_tmp_bytes, "scan temp")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&pos_out, cap * D * sizeof(float), "positions")) != MPM_OK) return rc;
 
     e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
@@ -756,7 +754,7 @@ void Engine::release() {
     }
     void* ptrs[] = {groups_d, scenes_d, grid_mom, grid_vel, err_d, keys[0], keys[1], vals[0], vals[1],
                     cell_count, seg_count, seg_start, sort_tmp, blk_flag, active, blk_epoch, counters, chunks,
-                    scan_tmp, pos_out, cell_end, det_src, det_sorted, det_blocks, det_runs, det_partial,
+                    pos_out, cell_end, det_src, det_sorted, det_blocks, det_runs, det_partial,
                     sur_counts, speed_max, scene_time,
                     pages.page, pages.slot_block, pages.free_slots};
     for (void* p : ptrs) cudaFree(p);
@@ -777,7 +775,6 @@ void Engine::release() {
     blk_flag = nullptr;
     active = blk_epoch = counters = nullptr;
     chunks = nullptr;
-    scan_tmp = nullptr;
     pos_out = nullptr;
     if (copy_stream) cudaStreamSynchronize(copy_stream);
     for (auto& sl : pos_slots) {
@@ -809,6 +806,22 @@ void Engine::drop_graphs() {
 }
 
 // ---------------------------------------------------------- launches --
+
+// launch attributes of a kernel that calls pdl_wait before it reads what the
+// kernel ahead of it wrote (programmatic dependent launch)
+static cudaLaunchConfig_t pdl_config(unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                                     cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return c;
+}
 
 void Engine::enqueue_direct_substep() {
     const ParticleBuf pb = buf(cur);
@@ -845,7 +858,6 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
     // next one rewrites, stay behind
     const bool reclaim = in_loop;
     const int to = 1 - from;
-    const long long n_segs = total_blocks * 4;
     int* rank = reinterpret_cast<int*>(vals[0]);
     if (paged && reclaim) {
         // blocks with nothing active near them give their physical block back
@@ -854,47 +866,48 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
                                                           (int)scenes_h.size());
         note_launch("k_pool_reclaim");
     }
-    cudaMemsetAsync(counters + CNT_CHUNKS, 0, kMats * sizeof(int), stream);
+    if (n_particles == 0) {  // the chunk lists stay empty
+        k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_REBINS);
+        note_launch("k_count_rebin");
+        sorted_order = true;
+        return;
+    }
+    const BinCounters bc{counters + CNT_CHUNKS, counters + CNT_PLACED, counters + CNT_REBINS};
     const unsigned nb = grid_blocks(n_particles, 256);
-    if (n_particles > 0) {
-        // the particles arrive in the order the configuration's last binning gave them
-        const bool cm = kFusedCfgs[cfg].order == ORDER_CELL;
+    // the particles arrive in the order the configuration's last binning gave them
+    const bool cm = kFusedCfgs[cfg].order == ORDER_CELL;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t lc = pdl_config(nb, 256, 0, stream, &attr);
+    {
         auto k = dim == 3 ? (paged ? (cm ? k_bin_count<3, true, true> : k_bin_count<3, true, false>)
                                    : (cm ? k_bin_count<3, false, true> : k_bin_count<3, false, false>))
                           : (paged ? (cm ? k_bin_count<2, true, true> : k_bin_count<2, true, false>)
                                    : (cm ? k_bin_count<2, false, true> : k_bin_count<2, false, false>));
-        k<<<nb, 256, 0, stream>>>(buf(from), n_particles, groups_d, scenes_d, mat_slots, keys[0], rank, cell_count,
-                                  seg_count, pages);
-        note_launch("k_bin_count");
+        note_launch_status("k_bin_count",
+                           cudaLaunchKernelEx(&lc, k, buf(from), n_particles, (const GroupParams*)groups_d,
+                                              (const SceneParams*)scenes_d, mat_slots, keys[0], rank, cell_count,
+                                              seg_count, pages, bc));
     }
-    cub::DeviceScan::ExclusiveSum(scan_tmp, scan_tmp_bytes, seg_count, seg_start, (int)n_segs, stream);
-    note_launch("cub::DeviceScan::ExclusiveSum");
-    if (n_particles > 0) {
-        const bool cm = kFusedCfgs[cfg].order == ORDER_CELL;
+    lc.gridDim = dim3(grid_blocks(total_blocks, 256));
+    note_launch_status("k_bin_segments",
+                       cudaLaunchKernelEx(&lc, dim == 3 ? k_bin_segments<3> : k_bin_segments<2>,
+                                          reinterpret_cast<const int4*>(seg_count), reinterpret_cast<int4*>(seg_start),
+                                          total_blocks, chunks, list_cap, bc, chunk_particles(),
+                                          (const SceneParams*)scenes_d, (int)scenes_h.size(), err_d));
+    lc.gridDim = dim3(nb);
+    {
         auto k = dim == 3 ? (paged ? (cm ? k_bin_place<3, true, true> : k_bin_place<3, true, false>)
                                    : (cm ? k_bin_place<3, false, true> : k_bin_place<3, false, false>))
                           : (paged ? (cm ? k_bin_place<2, true, true> : k_bin_place<2, true, false>)
                                    : (cm ? k_bin_place<2, false, true> : k_bin_place<2, false, false>));
-        k<<<nb, 256, 0, stream>>>(buf(from), buf(to), n_particles, keys[0], rank, cell_count, seg_count, seg_start,
-                                  mat_slots, in_loop ? 0 : 1, err_d, pages);
-        note_launch("k_bin_place");
+        note_launch_status("k_bin_place",
+                           cudaLaunchKernelEx(&lc, k, buf(from), buf(to), n_particles, (const unsigned long long*)keys[0],
+                                              (const int*)rank, (const int*)cell_count, (const int*)seg_count,
+                                              (const int*)seg_start, mat_slots, in_loop ? 0 : 1, err_d, pages));
     }
-    if (dim == 3)
-        k_make_chunks<3><<<grid_blocks(n_segs, 256), 256, 0, stream>>>(seg_count, seg_start, n_segs, chunks, list_cap,
-                                                                       counters + CNT_CHUNKS, chunk_particles(),
-                                                                       scenes_d, (int)scenes_h.size(), err_d);
-    else
-        k_make_chunks<2><<<grid_blocks(n_segs, 256), 256, 0, stream>>>(seg_count, seg_start, n_segs, chunks, list_cap,
-                                                                       counters + CNT_CHUNKS, chunk_particles(),
-                                                                       scenes_d, (int)scenes_h.size(), err_d);
-    note_launch("k_make_chunks");
-    if (n_particles > 0) {
-        auto k = paged ? k_bin_reset<true> : k_bin_reset<false>;
-        k<<<nb, 256, 0, stream>>>(keys[0], n_particles, mat_slots, cell_count, seg_count, pages);
-        note_launch("k_bin_reset");
-    }
-    k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_REBINS);
-    note_launch("k_count_rebin");
+    lc.gridDim = dim3(grid_blocks(total_blocks * 4, 256));
+    note_launch_status("k_bin_reset", cudaLaunchKernelEx(&lc, paged ? k_bin_reset<true> : k_bin_reset<false>,
+                                                         total_blocks * 4, mat_slots, cell_count, seg_count, pages));
     sorted_order = true;
 }
 
@@ -959,22 +972,6 @@ FusedArgs Engine::fused_args(int mat, bool bump) {
     A.pages = pages;
     A.vel_map = vel_map;
     return A;
-}
-
-// launch attributes of a kernel that calls pdl_wait before it reads what the
-// kernel ahead of it wrote (programmatic dependent launch)
-static cudaLaunchConfig_t pdl_config(unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
-                                     cudaLaunchAttribute* attr) {
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(block);
-    c.dynamicSmemBytes = smem;
-    c.stream = stream;
-    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr->val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = attr;
-    c.numAttrs = 1;
-    return c;
 }
 
 void Engine::enqueue_grid_update() {

@@ -70,8 +70,6 @@ struct Engine {
     int* seg_start = nullptr;
     void* sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
-    void* scan_tmp = nullptr;
-    size_t scan_tmp_bytes = 0;
     Chunk* chunks = nullptr;    // kMats lists of list_cap entries
     long long list_cap = 0;
     bool mat_present[3] = {false, false, false};

@@ -62,6 +62,14 @@ struct TileShape<2> {
     static constexpr bool SWIZZLE = false;
 };
 
+// Programmatic dependent launch: a kernel launched with programmatic stream
+// serialization may start before the kernel ahead of it in the stream ends;
+// pdl_wait blocks until that kernel has completed and its writes are visible
+// (immediately when launched without the attribute), pdl_trigger lets the
+// next kernel in the stream begin launching.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // ------------------------------------------------------------- binning --
 
 template <int D>
@@ -87,6 +95,18 @@ __device__ __forceinline__ void home_of(const SceneParams& sc, const float* x, l
 // lanes of a warp sit in distinct cells) or cell-major (cells ascending, a
 // cell's particles together).
 
+// device counters of a re-binning: chunk list lengths per material, particles
+// given a segment so far, re-binnings
+struct BinCounters {
+    int* n_chunks;
+    int* placed;
+    int* rebins;
+};
+
+// The four kernels of a re-binning (count, segments, place, reset) are chained
+// by programmatic dependent launch; each waits for the one ahead before its
+// first access, whatever its threads do after, so the chain is transitive.
+//
 // Pass 1: home block b, cell c and material m of every particle, its rank
 // among the particles of (b, m, c) and the size of segment (b, m).
 // (PAGED: the cell counters of a block live at its physical block.)  The
@@ -101,8 +121,15 @@ __global__ void __launch_bounds__(256) k_bin_count(ParticleBuf pb, long long n, 
                                                    const SceneParams* __restrict__ scenes, MatSlots ms,
                                                    unsigned long long* __restrict__ key, int* __restrict__ rank,
                                                    int* __restrict__ cell_count, int* __restrict__ seg_count,
-                                                   GridPages gp) {
+                                                   GridPages gp, BinCounters bc) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {  // the counters of the kernels behind this one
+        for (int m = 0; m < kMats; ++m) bc.n_chunks[m] = 0;
+        *bc.placed = 0;
+        *bc.rebins += 1;
+    }
     if (i >= n) return;
     float x[D];
 #pragma unroll
@@ -130,7 +157,7 @@ __global__ void __launch_bounds__(256) k_bin_count(ParticleBuf pb, long long n, 
     key[i] = ((unsigned long long)b << 8) | ((unsigned long long)g.type << 6) | (unsigned long long)c;
 }
 
-// Pass 2 (after the scan of the segment sizes): with n_c' the segment's cell
+// Pass 3 (after the segments have their places): with n_c' the segment's cell
 // counts, the slot of particle (r, c) in its segment is, rank-major,
 //   sum over cells c' of min(n_c', r)   (particles of lower rank)
 // + #{c' < c : n_c' > r}                (rank r in lower cells),
@@ -146,6 +173,8 @@ __global__ void __launch_bounds__(256) k_bin_place(ParticleBuf src, ParticleBuf 
                                                    const int* __restrict__ seg_count,
                                                    const int* __restrict__ seg_start, MatSlots ms,
                                                    int move_vc, unsigned* __restrict__ err, GridPages gp) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned long long k = key[i];
@@ -186,52 +215,86 @@ __device__ __forceinline__ void tile_origin(const SceneParams& sc, long long lb,
     o[2] = (D == 3) ? (int)(lb / ((long long)sc.nb[0] * sc.nb[1])) * SIDE - 1 : 0;
 }
 
-// one chunk per `chunk` particles of every non-empty (block, material)
-// segment, appended to that material's list, with its scene and window
-// origin (the block's coordinates, divided out once here)
+// Pass 2, a thread per block: the place of each of its segments in the ordered
+// state -- a CTA's 256 blocks follow one another, CTAs in the order they reach
+// the counter -- and one chunk per `chunk` particles of every non-empty
+// segment, appended to its material's list, with its scene and window origin
+// (the block's coordinates, divided out once here).
 template <int D>
-__global__ void __launch_bounds__(256) k_make_chunks(const int* __restrict__ seg_count,
-                                                     const int* __restrict__ seg_start, long long n_segs,
-                                                     Chunk* __restrict__ chunks, long long list_cap,
-                                                     int* __restrict__ n_chunks, int chunk,
-                                                     const SceneParams* __restrict__ scenes, int n_scenes,
-                                                     unsigned* __restrict__ err) {
-    const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_segs) return;
-    const int c = seg_count[s];
-    if (c == 0) return;
-    const int mat = (int)(s & 3);
-    const int nch = (c + chunk - 1) / chunk;
-    const int at = atomicAdd(&n_chunks[mat], nch);
-    if (at + nch > list_cap) {  // cannot happen with the list sized for the smallest chunk
-        atomicOr(err, ERR_BINNING);
-        return;
+__global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ seg_count, int4* __restrict__ seg_start,
+                                                      long long n_blocks, Chunk* __restrict__ chunks, long long list_cap,
+                                                      BinCounters bc, int chunk, const SceneParams* __restrict__ scenes,
+                                                      int n_scenes, unsigned* __restrict__ err) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ int warp_sum[8];
+    __shared__ int cta_start;
+    const long long b = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int4 c4 = b < n_blocks ? seg_count[b] : make_int4(0, 0, 0, 0);
+    const int c[4] = {c4.x, c4.y, c4.z, c4.w};
+    const int mine = c[0] + c[1] + c[2] + c[3];
+    int incl = mine;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, k);
+        if (lane >= k) incl += up;
     }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int w = 0; w < 8; ++w) {
+            const int v = warp_sum[w];
+            warp_sum[w] = sum;
+            sum += v;
+        }
+        cta_start = sum ? atomicAdd(bc.placed, sum) : 0;
+    }
+    __syncthreads();
+    if (mine == 0) return;
+    const int start = cta_start + warp_sum[warp] + incl - mine;
+    const int at0[4] = {start, start + c[0], start + c[0] + c[1], start + c[0] + c[1] + c[2]};
+    seg_start[b] = make_int4(at0[0], at0[1], at0[2], at0[3]);
     Chunk ch;
-    ch.block = (int)(s >> 2);
-    ch.mat = mat;
-    ch.scene = scene_of_block(scenes, n_scenes, ch.block);
-    const SceneParams& sc = scenes[ch.scene];
-    tile_origin<D>(sc, ch.block - sc.block_off, ch.o);
-    for (int j = 0; j < nch; ++j) {
-        ch.start = seg_start[s] + j * chunk;
-        ch.count = min(chunk, c - j * chunk);
-        chunks[mat * list_cap + at + j] = ch;
+    ch.block = (int)b;
+    ch.scene = scene_of_block(scenes, n_scenes, b);
+    tile_origin<D>(scenes[ch.scene], b - scenes[ch.scene].block_off, ch.o);
+#pragma unroll
+    for (int m = 0; m < kMats; ++m) {
+        if (c[m] == 0) continue;
+        const int nch = (c[m] + chunk - 1) / chunk;
+        const int at = atomicAdd(&bc.n_chunks[m], nch);
+        if (at + nch > list_cap) {  // cannot happen with the list sized for the smallest chunk
+            atomicOr(err, ERR_BINNING);
+            continue;
+        }
+        ch.mat = m;
+        for (int j = 0; j < nch; ++j) {
+            ch.start = at0[m] + j * chunk;
+            ch.count = min(chunk, c[m] - j * chunk);
+            chunks[m * list_cap + at + j] = ch;
+        }
     }
 }
 
-// zero the cell and segment counters that k_bin_count touched
+// Pass 4: zeroes the counters that pass 1 touched, a thread per segment; a
+// non-empty segment's 64 cell counters by its warp
 template <bool PAGED>
-__global__ void __launch_bounds__(256) k_bin_reset(const unsigned long long* __restrict__ key, long long n,
-                                                   MatSlots ms, int* __restrict__ cell_count,
+__global__ void __launch_bounds__(256) k_bin_reset(long long n_segs, MatSlots ms, int* __restrict__ cell_count,
                                                    int* __restrict__ seg_count, GridPages gp) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long k = key[i];
-    const long long b = (long long)(k >> 8);
-    const int m = (int)((k >> 6) & 3);
-    cell_count[(phys_block<PAGED>(gp, b) * ms.n + ms.s[m]) * 64 + (int)(k & 63)] = 0;
-    seg_count[b * 4 + m] = 0;
+    pdl_wait();
+    pdl_trigger();
+    const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool used = s < n_segs && seg_count[s] != 0;
+    const int lane = threadIdx.x & 31;
+    const long long first = s - lane;  // the warp's first segment
+    for (unsigned todo = __ballot_sync(0xffffffffu, used); todo; todo &= todo - 1) {
+        const long long q = first + __ffs(todo) - 1;
+        int2* cells = reinterpret_cast<int2*>(cell_count + (phys_block<PAGED>(gp, q >> 2) * ms.n + ms.s[q & 3]) * 64);
+        cells[lane] = make_int2(0, 0);
+    }
+    if (used) seg_count[s] = 0;
 }
 
 static __global__ void k_count_rebin(int* counter) { *counter += 1; }
@@ -391,16 +454,7 @@ __global__ void __launch_bounds__(256) k_pool_reclaim(GridPages gp, const unsign
 
 // Grid update of the active blocks: velocity into grid_vel, momentum buffer
 // cleared for the next P2G, block flag reset, block epoch stamped.
-// 64 threads per block, 4 blocks per CTA, persistent over the list.
-// Programmatic dependent launch: a kernel launched with programmatic stream
-// serialization may start before the kernel ahead of it in the stream ends;
-// pdl_wait blocks until that kernel has completed and its writes are visible
-// (immediately when launched without the attribute), pdl_trigger lets the
-// next kernel in the stream begin launching.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
-// Grid update of the blocks P2G touched.  The last CTA to finish resets the
+// 64 threads per block, 4 blocks per CTA, persistent over the list.  The last CTA to finish resets the
 // active-block count and the fused kernels' chunk cursors for the next pass
 // (every CTA has read the count before it counts itself done).
 // FIXED: the one scene of a fixed-dt run comes from the kernel parameters
