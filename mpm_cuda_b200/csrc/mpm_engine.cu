@@ -524,6 +524,10 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
 
 int Engine::chunk_particles() const { return kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds; }
 
+// the learned-stress kernel's shared memory leaves no room for the extra warp
+// of particles (3 instead of 4 CTAs per SM)
+int Engine::chunk_cap() const { return sur ? chunk_particles() : chunk_capacity(cfg, paged); }
+
 void Engine::set_config(int ci) {
     cfg = ci;
     const int dyn = fused_dyn_smem(dim, ci, paged);
@@ -557,7 +561,6 @@ void Engine::set_config(int ci) {
 // CTAs measured slower), else 64; it takes ceil(chunk_particles() / that)
 // rounds, the last one partly idle when the chunk is not a multiple of it
 int Engine::sur_chunk() const { return chunk_particles() >= 128 ? 128 : 64; }
-int Engine::sur_rounds() const { return (chunk_particles() + sur_chunk() - 1) / sur_chunk(); }
 
 void Engine::sur_occupancy() {
     for (int mat = 0; mat < kMats; ++mat) {
@@ -568,10 +571,10 @@ void Engine::sur_occupancy() {
         // window and weights they exceed the 48 KB a kernel gets without opting
         // in (the limit is the function's: always the largest chunk's)
         if (cudaFuncSetAttribute(sur_fn(ch, fixed_scene, paged), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 sur_dyn_smem(ch, ch == 64 ? 1 : kSurMaxRounds)) != cudaSuccess)
+                                 sur_dyn_smem_max(ch)) != cudaSuccess)
             cudaGetLastError();  // not fatal here: the occupancy query and the launch report it
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sur_fn(ch, fixed_scene, paged), ch,
-                                                          sur_dyn_smem(ch, sur_rounds())) != cudaSuccess) {
+                                                          sur_dyn_smem(ch, chunk_cap())) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 1;
         }
@@ -893,6 +896,7 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
                        cudaLaunchKernelEx(&lc, dim == 3 ? k_bin_segments<3> : k_bin_segments<2>,
                                           reinterpret_cast<const int4*>(seg_count), reinterpret_cast<int4*>(seg_start),
                                           total_blocks, chunks, list_cap, bc, chunk_particles(),
+                                          chunk_cap(),
                                           (const SceneParams*)scenes_d, (int)scenes_h.size(), err_d));
     lc.gridDim = dim3(nb);
     {
@@ -960,6 +964,7 @@ FusedArgs Engine::fused_args(int mat, bool bump) {
     A.fallback = (unsigned*)(counters + CNT_FALLBACK);
     A.speed_max = opt.adaptive_dt ? speed_max : nullptr;
     A.rounds = kFusedCfgs[cfg].rounds;
+    A.chunk_cap = chunk_cap();
     A.defer_vc = defer_vc_now() ? 1 : 0;
     A.scene = scenes_h[0];
     // the material's only group, when it has one
@@ -1002,11 +1007,9 @@ void Engine::enqueue_g2p2g(int parity) {
         if (sur_kernel(mat)) {
             const SurArgs SA{&sur->weights->f, sur->meta, sur_counts};
             const int ch = sur_chunk();
-            FusedArgs As = A;
-            As.rounds = sur_rounds();
             cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t lc = pdl_config(sur_ctas[mat], ch, sur_dyn_smem(ch, As.rounds), stream, &attr);
-            const cudaError_t e = cudaLaunchKernelEx(&lc, sur_fn(ch, fixed_scene, paged), buf(parity), As, SA);
+            const cudaLaunchConfig_t lc = pdl_config(sur_ctas[mat], ch, sur_dyn_smem(ch, A.chunk_cap), stream, &attr);
+            const cudaError_t e = cudaLaunchKernelEx(&lc, sur_fn(ch, fixed_scene, paged), buf(parity), A, SA);
             note_launch_status("k_g2p2g_sur", e);
         } else {
             cudaLaunchAttribute attr;
@@ -1701,6 +1704,7 @@ int Engine::set_stress_mode(int mode, Surrogate* s) {
     sur_version = sur ? sur->version : -1;
     sur_occupancy();
     drop_graphs();
+    steps_since_rebin = opt.rebin_interval;  // the next substep re-bins: the chunks' size depends on the mode
     return MPM_OK;
 }
 

@@ -94,6 +94,7 @@ struct Engine {
     int cfg = 1;                     // index into kFusedCfgs
     // particles per chunk of the current configuration (CTA size x rounds)
     int chunk_particles() const;
+    int chunk_cap() const;
     bool fixed_scene = false;        // one scene, fixed dt: fused kernels take it as a parameter
     // paged grid (mpm_options.grid_pool_blocks > 0): the grid arrays hold
     // pool_cap physical blocks plus the trash block; `pages` points at the
@@ -191,7 +192,6 @@ struct Engine {
     bool sur_kernel(int mat) const { return sur && dim == 3 && mat == JELLO; }
     void sur_occupancy();
     int sur_chunk() const;
-    int sur_rounds() const;
     int sur_refresh();
     void enqueue_det_p2g();
     void enqueue_det_substep();

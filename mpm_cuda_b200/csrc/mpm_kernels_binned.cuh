@@ -223,7 +223,8 @@ __device__ __forceinline__ void tile_origin(const SceneParams& sc, long long lb,
 template <int D>
 __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ seg_count, int4* __restrict__ seg_start,
                                                       long long n_blocks, Chunk* __restrict__ chunks, long long list_cap,
-                                                      BinCounters bc, int chunk, const SceneParams* __restrict__ scenes,
+                                                      BinCounters bc, int chunk, int chunk_cap,
+                                                      const SceneParams* __restrict__ scenes,
                                                       int n_scenes, unsigned* __restrict__ err) {
     pdl_wait();
     pdl_trigger();
@@ -263,7 +264,10 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
 #pragma unroll
     for (int m = 0; m < kMats; ++m) {
         if (c[m] == 0) continue;
-        const int nch = (c[m] + chunk - 1) / chunk;
+        // as few chunks as hold the segment, of `chunk` particles, or of equal
+        // shares where those would leave a rest
+        const int nch = (c[m] + chunk_cap - 1) / chunk_cap;
+        const int size = max(chunk, (c[m] + nch - 1) / nch);
         const int at = atomicAdd(&bc.n_chunks[m], nch);
         if (at + nch > list_cap) {  // cannot happen with the list sized for the smallest chunk
             atomicOr(err, ERR_BINNING);
@@ -271,8 +275,8 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
         }
         ch.mat = m;
         for (int j = 0; j < nch; ++j) {
-            ch.start = at0[m] + j * chunk;
-            ch.count = min(chunk, c[m] - j * chunk);
+            ch.start = at0[m] + j * size;
+            ch.count = min(size, c[m] - j * size);
             chunks[m * list_cap + at + j] = ch;
         }
     }
@@ -542,6 +546,7 @@ struct FusedArgs {
     unsigned* fallback;  // count of particles that used global memory
     unsigned* speed_max; // adaptive dt: per scene max of |v| + wave (float bits); null when off
     int rounds;          // particles per thread and chunk (a chunk holds CTA size x rounds)
+    int chunk_cap;       // most particles a chunk holds (run sums)
     int defer_vc;        // store the pre-advection position in the v planes and no C (k_recover_vc)
     // the one scene of a single-scene run with a fixed dt, read by the kernels
     // built with FIXED = true from their parameters (constant bank operands,

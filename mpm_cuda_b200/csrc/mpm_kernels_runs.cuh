@@ -185,10 +185,11 @@ __device__ __forceinline__ void sum_plane2(const float4* __restrict__ recs, int 
 template <int D>
 struct __align__(128) RunShared {
     float4 tv[TileShape<D>::VN];      // the chunk's velocity window
-    int hist[kRunBins];               // runs per length, longest first
     Chunk ch[2];                      // records of this and the next chunk
     int head[2][RunShape<D>::N];      // first record of each base's run, -1: none
     int cnt[RunShape<D>::N];          // its length, reset by its reader
+    int level[2][kRunBins];           // runs longer than k
+    int taken[kRunBins];              // runs of a length given a place so far
     int s27[2][27];                   // PAGED: the windows' physical blocks
     int n_runs[2];
     unsigned touched[2];              // 3^D neighbour-block bits
@@ -208,13 +209,16 @@ __device__ __forceinline__ void insert_record(RunShared<D>& sm, float4* recs, un
         const int l0 = sn.base[0] - o[0], l1 = sn.base[1] - o[1], l2 = D == 3 ? sn.base[2] - o[2] : 0;
         const int key = l0 + RS::B * (l1 + RS::B * l2);
         next = atomicExch(&sm.head[b][key], li);
-        atomicAdd(&sm.cnt[key], 1);
+        // the run now has more than `longer` records; one record of a run says so
+        const int longer = atomicAdd(&sm.cnt[key], 1);
+        if (longer < kRunBins) atomicAdd(&sm.level[b][longer], 1);
         if (next < 0) {
             runs[atomicAdd(&sm.n_runs[b], 1)] = (unsigned short)key;
             atomicOr(&sm.touched[b], touched_bits<D>(l0, l1, l2));
         }
     } else {
         atomicAdd(A.fallback, 1u);
+        atomicAdd(&sm.level[b][0], 1);
         runs[atomicAdd(&sm.n_runs[b], 1)] = (unsigned short)(kRunOutside | (unsigned)li);
     }
     write_record<D>(recs + li * run_rec4(D), sn, src, sc.h, sc.inv_h, next);
@@ -229,19 +233,19 @@ __device__ __forceinline__ void load_position(const ParticleBuf& pb, long long i
 // The pass of a CTA over its chunks.  round(ch, sc, o, b, li, x, speed_bits) is
 // phase A of one particle of every thread (li >= ch.count: none), at position x
 // (the round may overwrite it); it puts the
-// P2G source it computes on the lists of parity b with insert_record.  A chunk
-// holds at most CHUNK x MAXR particles.
-template <int D, int CHUNK, int MAXR, bool FIXED, bool PAGED, class Round>
+// P2G source it computes on the lists of parity b with insert_record.
+template <int D, int CHUNK, bool FIXED, bool PAGED, class Round>
 __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArgs& A, RunShared<D>& sm, float4* recs,
                                            unsigned short* runs, Round round) {
     using P = Planes<D>;
     using RS = RunShape<D>;
     constexpr bool TMA = FIXED && !PAGED;
+    unsigned short* sorted = runs + A.chunk_cap;
     for (int t = threadIdx.x; t < RS::N; t += CHUNK) {
         sm.head[0][t] = sm.head[1][t] = -1;
         sm.cnt[t] = 0;
     }
-    if (threadIdx.x < kRunBins) sm.hist[threadIdx.x] = 0;
+    if (threadIdx.x < kRunBins) sm.level[0][threadIdx.x] = sm.level[1][threadIdx.x] = sm.taken[threadIdx.x] = 0;
     if (threadIdx.x < 2) {
         sm.n_runs[threadIdx.x] = 0;
         sm.touched[threadIdx.x] = 0u;
@@ -292,7 +296,7 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
         const int o[3] = {ch.o[0], ch.o[1], ch.o[2]};
         unsigned speed_bits = 0u;
 #pragma unroll 1
-        for (int r = 0; r < A.rounds; ++r) {
+        for (int r = 0; r * CHUNK < ch.count; ++r) {
             const int li = (int)threadIdx.x + r * CHUNK;
             if (r > 0 && li < ch.count) load_position<D>(pb, (long long)ch.start + li, x);
             round(ch, sc, o, b, li, x, speed_bits);
@@ -324,40 +328,28 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
         }
         // the runs by length, the longest first, so that the lanes of a warp
         // walk runs of about one length: a run's place is the number of longer
-        // runs plus its rank among those of its length
+        // runs, counted as the records came in, plus its turn among those of its
+        // length (those of kRunBins or more together)
         const int nr = sm.n_runs[b];
-        unsigned entry[MAXR];
-        int bin[MAXR], rank[MAXR];
-#pragma unroll
-        for (int q = 0; q < MAXR; ++q) {
-            const int t = (int)threadIdx.x + q * CHUNK;
-            if (t < nr) {
-                entry[q] = runs[t];
-                int len = 1;
-                if (!(entry[q] & kRunOutside)) {
-                    len = sm.cnt[entry[q]];
-                    sm.cnt[entry[q]] = 0;
-                }
-                bin[q] = kRunBins - min(len, kRunBins);
-                rank[q] = atomicAdd(&sm.hist[bin[q]], 1);
+        if (threadIdx.x < kRunBins) sm.level[b ^ 1][threadIdx.x] = 0;
+        for (int t = threadIdx.x; t < nr; t += CHUNK) {
+            const unsigned e = runs[t];
+            int len = 1;
+            if (!(e & kRunOutside)) {
+                len = sm.cnt[e];
+                sm.cnt[e] = 0;
             }
+            const int k = min(len, kRunBins) - 1;
+            const int longer = k + 1 < kRunBins ? sm.level[b][k + 1] : 0;
+            sorted[longer + atomicAdd(&sm.taken[k], 1)] = (unsigned short)e;
         }
         __syncthreads();  // (3)
-#pragma unroll
-        for (int q = 0; q < MAXR; ++q) {
-            if ((int)threadIdx.x + q * CHUNK < nr) {
-                int at = rank[q];
-                for (int j = 0; j < bin[q]; ++j) at += sm.hist[j];
-                runs[at] = (unsigned short)entry[q];
-            }
-        }
-        __syncthreads();  // (4)
-        if (threadIdx.x < kRunBins) sm.hist[threadIdx.x] = 0;
+        if (threadIdx.x < kRunBins) sm.taken[threadIdx.x] = 0;
         // ---- phase B
         const int items = nr * RS::PLANES;
         for (int it = threadIdx.x; it < items; it += CHUNK) {
             const int run = D == 3 ? it / 3 : it, ox = D == 3 ? it - 3 * run : 0;
-            const unsigned e = runs[run];
+            const unsigned e = sorted[run];
             int base[3] = {o[0], o[1], o[2]};
             int slot;
             if (e & kRunOutside) {
@@ -422,10 +414,10 @@ template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
     __shared__ RunShared<D> sm;
     extern __shared__ __align__(16) float4 recs[];
-    unsigned short* runs = reinterpret_cast<unsigned short*>(recs + CHUNK * A.rounds * run_rec4(D));
-    run_chunks<D, CHUNK, kMaxRunRounds, FIXED, PAGED>(pb, A, sm, recs, runs,
-                                                      [&](const Chunk& ch, const SceneParams& sc, const int* o, int b,
-                                                          int li, float* x, unsigned& speed_bits) {
+    unsigned short* runs = reinterpret_cast<unsigned short*>(recs + A.chunk_cap * run_rec4(D));
+    run_chunks<D, CHUNK, FIXED, PAGED>(pb, A, sm, recs, runs,
+                                       [&](const Chunk& ch, const SceneParams& sc, const int* o, int b, int li, float* x,
+                                           unsigned& speed_bits) {
         if (li >= ch.count) return;
         const long long i = (long long)ch.start + li;
         float* S = pb.s;

@@ -28,12 +28,18 @@ namespace mpm {
 // BF16 features, then 9 outputs; odd, so the rows of a warp's 32 particles
 // start in 32 different banks
 constexpr int kSurRowStride = 9;
-// particles per thread of a chunk at most (512-particle chunks)
-constexpr int kSurMaxRounds = 4;
 // dynamic shared memory of k_g2p2g_sur: the chunk's records and run list, a
 // network row per thread
-constexpr int sur_dyn_smem(int cta, int rounds) {
-    return run_smem(3, cta * rounds) + cta * kSurRowStride * (int)sizeof(float);
+constexpr int sur_dyn_smem(int cta, int particles) {
+    return run_smem(3, particles) + cta * kSurRowStride * (int)sizeof(float);
+}
+// the most any configuration asks for
+constexpr int sur_dyn_smem_max(int cta) {
+    int most = 0;
+    for (int i = 0; i < kNumFusedCfgs; ++i)
+        for (int paged = 0; paged < 2; ++paged)
+            most = chunk_capacity(i, paged != 0) > most ? chunk_capacity(i, paged != 0) : most;
+    return sur_dyn_smem(cta, most);
 }
 
 struct SurArgs {
@@ -53,7 +59,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
     __shared__ RunShared<D> sm;
     __shared__ __align__(16) mlp::Forward W;  // network weights
     extern __shared__ __align__(16) float4 recs[];
-    float* rows = reinterpret_cast<float*>(recs + CHUNK * A.rounds * run_rec4(D));
+    float* rows = reinterpret_cast<float*>(recs + A.chunk_cap * run_rec4(D));
     unsigned short* runs = reinterpret_cast<unsigned short*>(rows + CHUNK * XS);
 
     {
@@ -66,9 +72,9 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_sur(ParticleBuf pb, const
     float* row = rows + threadIdx.x * XS;
     unsigned n_net = 0, n_svd = 0;
     // every thread runs every round (the network step is warp-synchronous)
-    run_chunks<D, CHUNK, kSurMaxRounds, FIXED, PAGED>(pb, A, sm, recs, runs,
-                                                      [&](const Chunk& ch, const SceneParams& sc, const int* o, int b,
-                                                          int li, float* x, unsigned& speed_bits) {
+    run_chunks<D, CHUNK, FIXED, PAGED>(pb, A, sm, recs, runs,
+                                       [&](const Chunk& ch, const SceneParams& sc, const int* o, int b, int li, float* x,
+                                           unsigned& speed_bits) {
         unsigned err = 0;
         bool next = false;      // the particle scatters into the next substep
         bool eligible = false;  // its group takes the network's stress
