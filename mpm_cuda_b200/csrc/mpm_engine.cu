@@ -31,18 +31,18 @@ constexpr int kDefaultRebinInterval = 16;
 // device counters: chunk list lengths and cursors per material, active
 // block count, grid epoch, tile fallbacks, re-binnings
 enum {
-    CNT_CHUNKS = 0,
-    CNT_ACTIVE = 3,
-    CNT_EPOCH = 4,
-    CNT_CURSOR = 5,
-    CNT_FALLBACK = 8,
-    CNT_REBINS = 9,
-    CNT_UPDATE_DONE = 10,
-    CNT_POOL_FREE = 11,  // paged grid: height of the free stack
-    CNT_DET_BLOCKS = 12, // deterministic P2G: length of the ascending list of marked blocks
-    CNT_DET_RUNS = 13,   // deterministic P2G: number of runs of records sharing a base node
-    CNT_PLACED = 14,     // re-binning: particles given a segment so far
-    CNT_N = 16
+    CNT_CHUNKS = 0,      // large chunks per material, then small ones
+    CNT_ACTIVE = 6,
+    CNT_EPOCH = 7,
+    CNT_CURSOR = 8,
+    CNT_FALLBACK = 11,
+    CNT_REBINS = 12,
+    CNT_UPDATE_DONE = 13,
+    CNT_POOL_FREE = 14,  // paged grid: height of the free stack
+    CNT_DET_BLOCKS = 15, // deterministic P2G: length of the ascending list of marked blocks
+    CNT_DET_RUNS = 16,   // deterministic P2G: number of runs of records sharing a base node
+    CNT_PLACED = 17,     // re-binning: particles given a segment so far
+    CNT_N = 32
 };
 
 // Where a state transfer keeps each field (x, v, C, F, aux) in its scratch
@@ -949,6 +949,7 @@ FusedArgs Engine::fused_args(int mat, bool bump) {
     FusedArgs A;
     A.chunks = chunks + mat * list_cap;
     A.n_chunks = counters + CNT_CHUNKS + mat;
+    A.list_cap = (int)list_cap;
     A.cursor = counters + CNT_CURSOR + mat;
     A.groups = groups_d;
     A.scenes = scenes_d;

@@ -95,8 +95,10 @@ __device__ __forceinline__ void home_of(const SceneParams& sc, const float* x, l
 // lanes of a warp sit in distinct cells) or cell-major (cells ascending, a
 // cell's particles together).
 
-// device counters of a re-binning: chunk list lengths per material, particles
-// given a segment so far, re-binnings
+// device counters of a re-binning: chunk list lengths per material (n_chunks[m]
+// chunks of at least half the nominal size from the front of the list,
+// n_chunks[kMats + m] smaller ones from its back), particles given a segment so
+// far, re-binnings
 struct BinCounters {
     int* n_chunks;
     int* placed;
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(256) k_bin_count(ParticleBuf pb, long long n, 
     pdl_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {  // the counters of the kernels behind this one
-        for (int m = 0; m < kMats; ++m) bc.n_chunks[m] = 0;
+        for (int m = 0; m < 2 * kMats; ++m) bc.n_chunks[m] = 0;
         *bc.placed = 0;
         *bc.rebins += 1;
     }
@@ -268,16 +270,19 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
         // shares where those would leave a rest
         const int nch = (c[m] + chunk_cap - 1) / chunk_cap;
         const int size = max(chunk, (c[m] + nch - 1) / nch);
-        const int at = atomicAdd(&bc.n_chunks[m], nch);
-        if (at + nch > list_cap) {  // cannot happen with the list sized for the smallest chunk
+        const int rest = c[m] - (nch - 1) * size;  // the last one's particles
+        const int large = rest * 2 >= chunk ? nch : nch - 1;
+        const int at = large ? atomicAdd(&bc.n_chunks[m], large) : 0;
+        const int back = large < nch ? atomicAdd(&bc.n_chunks[kMats + m], 1) : 0;
+        if (at + large > list_cap || back >= list_cap) {  // cannot happen with the list sized for the smallest chunk
             atomicOr(err, ERR_BINNING);
             continue;
         }
         ch.mat = m;
         for (int j = 0; j < nch; ++j) {
             ch.start = at0[m] + j * size;
-            ch.count = min(size, c[m] - j * size);
-            chunks[m * list_cap + at + j] = ch;
+            ch.count = j < nch - 1 ? size : rest;
+            chunks[m * list_cap + (j < large ? at + j : list_cap - 1 - back)] = ch;
         }
     }
 }
@@ -529,8 +534,9 @@ __global__ void __launch_bounds__(256) k_grid_update_active(float4* __restrict__
 // ------------------------------------------------------------ G2P2G --
 
 struct FusedArgs {
-    const Chunk* chunks;  // this material's chunk list
-    const int* n_chunks;  // its length
+    const Chunk* chunks;  // this material's chunk list: large ones from the front, small ones from the back
+    const int* n_chunks;  // how many large ones, and kMats words on how many small ones
+    int list_cap;
     int* cursor;          // next chunk to hand out (zeroed before every launch)
     const GroupParams* groups;
     const SceneParams* scenes;
@@ -563,6 +569,17 @@ struct FusedArgs {
     // FusedArgs as a __grid_constant__ parameter, so the copy engine reads the
     // map from the parameter space
     CUtensorMap vel_map;
+};
+
+// The c-th chunk a launch hands out: the large ones first, so that the small
+// ones fill the last wave
+struct ChunkList {
+    int large, all;
+    __device__ __forceinline__ explicit ChunkList(const FusedArgs& A)
+        : large(A.n_chunks[0]), all(A.n_chunks[0] + A.n_chunks[kMats]) {}
+    __device__ __forceinline__ const Chunk* at(const FusedArgs& A, int c) const {
+        return A.chunks + (c < large ? c : A.list_cap - 1 - (c - large));
+    }
 };
 
 // the group record of particle i of a fused launch
@@ -699,14 +716,14 @@ __device__ __forceinline__ void load_window(const FusedArgs& A, const Chunk& ch,
     }
 }
 
-// the same for chunk c of the list, keeping its record in *s_ch for the
+// the same for a chunk of the list, keeping its record in *s_ch for the
 // chunk's pass
 template <int D, int NT, bool FIXED, bool PAGED>
-__device__ __forceinline__ void prefetch_velocity_tile(const FusedArgs& A, int c, float4* tv, int* s27,
+__device__ __forceinline__ void prefetch_velocity_tile(const FusedArgs& A, const Chunk* chunk, float4* tv, int* s27,
                                                        Chunk* s_ch, unsigned long long* bar) {
     if constexpr (FIXED && !PAGED)
         if (threadIdx.x != 0) return;
-    const Chunk ch = A.chunks[c];
+    const Chunk ch = *chunk;
     if (threadIdx.x == 0) *s_ch = ch;
     load_window<D, NT, FIXED, PAGED>(A, ch, tv, s27, bar);
 }
@@ -948,7 +965,8 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
     // TMA: completion of window b's loads; window b's n-th load completes
     // phase n, so chunk k waits for parity (k >> 1) & 1 of barrier k & 1
     __shared__ __align__(8) unsigned long long s_bar[2];
-    const int nch = *A.n_chunks;
+    const ChunkList list(A);
+    const int nch = list.all;
     if (threadIdx.x == 0) {
         s_cn[0] = atomicAdd(A.cursor, 1);
         s_cn[1] = atomicAdd(A.cursor, 1);
@@ -961,12 +979,13 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
     __syncthreads();
     int cur = s_cn[0], nxt = s_cn[1];
     __syncthreads();  // s_cn is rewritten below
-    if (cur < nch) prefetch_velocity_tile<D, NT, FIXED, PAGED>(A, cur, tv[0], s27[0], &s_ch[0], &s_bar[0]);
+    if (cur < nch) prefetch_velocity_tile<D, NT, FIXED, PAGED>(A, list.at(A, cur), tv[0], s27[0], &s_ch[0], &s_bar[0]);
     cp_async_commit();
     for (int k = 0; cur < nch; ++k) {
         const int b = k & 1;
         if (nxt < nch)
-            prefetch_velocity_tile<D, NT, FIXED, PAGED>(A, nxt, tv[b ^ 1], s27[b ^ 1], &s_ch[b ^ 1], &s_bar[b ^ 1]);
+            prefetch_velocity_tile<D, NT, FIXED, PAGED>(A, list.at(A, nxt), tv[b ^ 1], s27[b ^ 1], &s_ch[b ^ 1],
+                                                        &s_bar[b ^ 1]);
         cp_async_commit();
         // the chunk after next: thread 0 keeps the cursor's answer in a
         // register and publishes it before barrier (2), so the atomic's round

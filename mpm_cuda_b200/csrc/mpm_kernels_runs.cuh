@@ -262,10 +262,11 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
     // of another material's pass, which wait for it) have all passed their own
     // wait.  So the first chunk's record and positions are fetched before this
     // kernel's wait; velocities, cursors and block flags after it.
-    const int nch = *A.n_chunks;
+    const ChunkList list(A);
+    const int nch = list.all;
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
-    if (threadIdx.x == 0 && cur < nch) sm.ch[0] = A.chunks[cur];
+    if (threadIdx.x == 0 && cur < nch) sm.ch[0] = *list.at(A, cur);
     __syncthreads();  // the record, the barrier and the lists initialised
     pdl_wait();     // the grid update ahead of this launch has finished
     pdl_trigger();  // the next pass may launch; it waits for this one to end
@@ -302,7 +303,7 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
             round(ch, sc, o, b, li, x, speed_bits);
             // the next chunk's record, on its way while the rest of this phase runs
             if (r == 0 && threadIdx.x == 0 && nxt < nch) {
-                const char* from = reinterpret_cast<const char*>(&A.chunks[nxt]);
+                const char* from = reinterpret_cast<const char*>(list.at(A, nxt));
                 char* to = reinterpret_cast<char*>(&sm.ch[b ^ 1]);
                 cp_async16(to, from, true);
                 cp_async16(to + 16, from + 16, true);
