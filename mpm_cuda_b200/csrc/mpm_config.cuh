@@ -86,23 +86,13 @@ constexpr bool sums_runs(int cfg, bool paged) {
     return paged ? c.scatter == SCATTER_DIRECT && c.order == ORDER_CELL && c.chunk == 128 && c.min_ctas <= 5
                  : c.scatter == SCATTER_RUNS;
 }
-// Particles a chunk may hold.  A run-sum chunk takes up to a warp more than its
-// threads x rounds: a block of 512 cells x particles has a few more or less
-// after some motion, and a chunk of its own for the rest (15-19 % of the chunks
-// of the 2M-particle scenes had 32 particles or fewer) costs a window, three
-// barriers and a nearly idle CTA.  Not with one round: those configurations are
-// for scenes that leave SMs idle, where one more CTA beats one more round
-// (2D jello 9.7 against 11.2 us a substep).
-constexpr int chunk_capacity(int cfg, bool paged) {
-    return kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds + (sums_runs(cfg, paged) && kFusedCfgs[cfg].rounds > 1 ? 32 : 0);
-}
 // SCATTER_RUNS: float4s of a particle's source record, and the dynamic shared
 // memory of a chunk (a record and two run-list entries per particle)
 constexpr int run_rec4(int dim) { return dim == 3 ? 6 : 4; }
 constexpr int run_smem(int dim, int particles) { return particles * (run_rec4(dim) * 16 + 4); }
 // dynamic shared memory of a launch configuration
 constexpr int fused_dyn_smem(int dim, int cfg, bool paged) {
-    return sums_runs(cfg, paged) ? run_smem(dim, chunk_capacity(cfg, paged)) : 0;
+    return sums_runs(cfg, paged) ? run_smem(dim, kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds) : 0;
 }
 // the most any configuration of the same instantiation asks for
 constexpr int fused_dyn_smem_max(int dim, int cfg, bool paged) {

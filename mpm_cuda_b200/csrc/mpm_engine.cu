@@ -524,10 +524,6 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
 
 int Engine::chunk_particles() const { return kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds; }
 
-// the learned-stress kernel's shared memory leaves no room for the extra warp
-// of particles (3 instead of 4 CTAs per SM)
-int Engine::chunk_cap() const { return sur ? chunk_particles() : chunk_capacity(cfg, paged); }
-
 void Engine::set_config(int ci) {
     cfg = ci;
     const int dyn = fused_dyn_smem(dim, ci, paged);
@@ -574,7 +570,7 @@ void Engine::sur_occupancy() {
                                  sur_dyn_smem_max(ch)) != cudaSuccess)
             cudaGetLastError();  // not fatal here: the occupancy query and the launch report it
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sur_fn(ch, fixed_scene, paged), ch,
-                                                          sur_dyn_smem(ch, chunk_cap())) != cudaSuccess) {
+                                                          sur_dyn_smem(ch, chunk_particles())) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 1;
         }
@@ -896,7 +892,6 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
                        cudaLaunchKernelEx(&lc, dim == 3 ? k_bin_segments<3> : k_bin_segments<2>,
                                           reinterpret_cast<const int4*>(seg_count), reinterpret_cast<int4*>(seg_start),
                                           total_blocks, chunks, list_cap, bc, chunk_particles(),
-                                          chunk_cap(),
                                           (const SceneParams*)scenes_d, (int)scenes_h.size(), err_d));
     lc.gridDim = dim3(nb);
     {
@@ -965,7 +960,7 @@ FusedArgs Engine::fused_args(int mat, bool bump) {
     A.fallback = (unsigned*)(counters + CNT_FALLBACK);
     A.speed_max = opt.adaptive_dt ? speed_max : nullptr;
     A.rounds = kFusedCfgs[cfg].rounds;
-    A.chunk_cap = chunk_cap();
+    A.chunk_cap = chunk_particles();
     A.defer_vc = defer_vc_now() ? 1 : 0;
     A.scene = scenes_h[0];
     // the material's only group, when it has one
@@ -1705,7 +1700,6 @@ int Engine::set_stress_mode(int mode, Surrogate* s) {
     sur_version = sur ? sur->version : -1;
     sur_occupancy();
     drop_graphs();
-    steps_since_rebin = opt.rebin_interval;  // the next substep re-bins: the chunks' size depends on the mode
     return MPM_OK;
 }
 

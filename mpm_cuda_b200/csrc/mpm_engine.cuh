@@ -94,7 +94,6 @@ struct Engine {
     int cfg = 1;                     // index into kFusedCfgs
     // particles per chunk of the current configuration (CTA size x rounds)
     int chunk_particles() const;
-    int chunk_cap() const;
     bool fixed_scene = false;        // one scene, fixed dt: fused kernels take it as a parameter
     // paged grid (mpm_options.grid_pool_blocks > 0): the grid arrays hold
     // pool_cap physical blocks plus the trash block; `pages` points at the

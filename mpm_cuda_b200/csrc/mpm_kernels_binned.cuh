@@ -225,8 +225,7 @@ __device__ __forceinline__ void tile_origin(const SceneParams& sc, long long lb,
 template <int D>
 __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ seg_count, int4* __restrict__ seg_start,
                                                       long long n_blocks, Chunk* __restrict__ chunks, long long list_cap,
-                                                      BinCounters bc, int chunk, int chunk_cap,
-                                                      const SceneParams* __restrict__ scenes,
+                                                      BinCounters bc, int chunk, const SceneParams* __restrict__ scenes,
                                                       int n_scenes, unsigned* __restrict__ err) {
     pdl_wait();
     pdl_trigger();
@@ -266,11 +265,8 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
 #pragma unroll
     for (int m = 0; m < kMats; ++m) {
         if (c[m] == 0) continue;
-        // as few chunks as hold the segment, of `chunk` particles, or of equal
-        // shares where those would leave a rest
-        const int nch = (c[m] + chunk_cap - 1) / chunk_cap;
-        const int size = max(chunk, (c[m] + nch - 1) / nch);
-        const int rest = c[m] - (nch - 1) * size;  // the last one's particles
+        const int nch = (c[m] + chunk - 1) / chunk;
+        const int rest = c[m] - (nch - 1) * chunk;  // the last one's particles
         const int large = rest * 2 >= chunk ? nch : nch - 1;
         const int at = large ? atomicAdd(&bc.n_chunks[m], large) : 0;
         const int back = large < nch ? atomicAdd(&bc.n_chunks[kMats + m], 1) : 0;
@@ -280,8 +276,8 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
         }
         ch.mat = m;
         for (int j = 0; j < nch; ++j) {
-            ch.start = at0[m] + j * size;
-            ch.count = j < nch - 1 ? size : rest;
+            ch.start = at0[m] + j * chunk;
+            ch.count = j < nch - 1 ? chunk : rest;
             chunks[m * list_cap + (j < large ? at + j : list_cap - 1 - back)] = ch;
         }
     }
@@ -552,7 +548,7 @@ struct FusedArgs {
     unsigned* fallback;  // count of particles that used global memory
     unsigned* speed_max; // adaptive dt: per scene max of |v| + wave (float bits); null when off
     int rounds;          // particles per thread and chunk (a chunk holds CTA size x rounds)
-    int chunk_cap;       // most particles a chunk holds (run sums)
+    int chunk_cap;       // most particles a chunk holds
     int defer_vc;        // store the pre-advection position in the v planes and no C (k_recover_vc)
     // the one scene of a single-scene run with a fixed dt, read by the kernels
     // built with FIXED = true from their parameters (constant bank operands,

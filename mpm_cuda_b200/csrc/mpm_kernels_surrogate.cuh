@@ -37,8 +37,7 @@ constexpr int sur_dyn_smem(int cta, int particles) {
 constexpr int sur_dyn_smem_max(int cta) {
     int most = 0;
     for (int i = 0; i < kNumFusedCfgs; ++i)
-        for (int paged = 0; paged < 2; ++paged)
-            most = chunk_capacity(i, paged != 0) > most ? chunk_capacity(i, paged != 0) : most;
+        most = kFusedCfgs[i].chunk * kFusedCfgs[i].rounds > most ? kFusedCfgs[i].chunk * kFusedCfgs[i].rounds : most;
     return sur_dyn_smem(cta, most);
 }
 
