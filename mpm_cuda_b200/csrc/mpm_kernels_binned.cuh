@@ -736,12 +736,12 @@ __device__ __forceinline__ bool in_window(const int* base, const int* o) {
 // G2P of one particle from the window, or from global memory for a particle
 // that drifted out of it since the last re-binning (LIN: grid_vel in the
 // linear layout)
-template <int D, bool PAGED = false, bool LIN = false>
+template <int D, bool PAGED = false, bool LIN = false, bool UNROLL_Y = false>
 __device__ __forceinline__ void g2p_window(const Stencil<D>& st, const int* o, const float4* tv, const SceneParams& sc,
                                            const FusedArgs& A, G2PAcc<D>& acc) {
     if (in_window<D>(st.base, o)) {
         const int b0 = st.base[0] - o[0], b1 = st.base[1] - o[1], b2 = D == 3 ? st.base[2] - o[2] : 0;
-        g2p_gather<D>(st, sc.inv_h, [&](int ox, int oy, int oz) {
+        g2p_gather<D, UNROLL_Y>(st, sc.inv_h, [&](int ox, int oy, int oz) {
             return tv[tv_idx<D>(b0 + ox, b1 + oy, b2 + oz)];
         }, acc);
     } else if constexpr (PAGED) {
@@ -767,17 +767,21 @@ __device__ __forceinline__ void g2p_window(const Stencil<D>& st, const int* o, c
 // new state; x, v, Cn, F, aux hold it on return.  defer_vc: the v planes get
 // the pre-advection position instead of v, and C is not stored; k_recover_vc
 // rebuilds both from it and the grid velocities when they are read.
+// preloaded: F holds the particle's planes already.
 template <int D, int MAT>
 __device__ __forceinline__ unsigned update_and_store(const G2PAcc<D>& acc, const SceneParams& sc, const GroupParams& g,
                                                      float* __restrict__ S, long long cap, long long i, float* x,
                                                      float* v, float* Cn, float* F, float& aux,
-                                                     typename SnowKeep<D>::T* keep = nullptr, bool defer_vc = false) {
+                                                     typename SnowKeep<D>::T* keep = nullptr, bool defer_vc = false,
+                                                     bool preloaded = false) {
     using P = Planes<D>;
     aux = 1.f;
     if (MAT != JELLO) aux = S[P::AUX * cap + i];
     if (MAT != WATER) {
+        if (!preloaded) {
 #pragma unroll
-        for (int k = 0; k < D * D; ++k) F[k] = S[(P::F + k) * cap + i];
+            for (int k = 0; k < D * D; ++k) F[k] = S[(P::F + k) * cap + i];
+        }
     } else {
 #pragma unroll
         for (int k = 0; k < D * D; ++k) F[k] = (k % (D + 1) == 0) ? 1.f : 0.f;

@@ -413,6 +413,15 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
 
 template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, const __grid_constant__ FusedArgs A) {
+    // What the registers allow, by measurement (substep, us; rolled gather / y
+    // loop unrolled / rolled with F loaded ahead of the gather).  128 registers:
+    // jello 256^3 214 / 212 / 206, snow 256^3 231 / 222 / 226, water tank 67.8 /
+    // 65.2 / -; scene table, 16 mixed scenes 255 / 242 / -.  96 registers: jello
+    // 211 / 228 / 224, snow 227 / 239 / 243, water 64.5 / 71.5 / -; scene table
+    // 241 / 233 / 244.
+    constexpr bool ROOMY = MINB <= 4;
+    constexpr bool PRELOAD = D == 3 && FIXED && ROOMY && MAT == JELLO;
+    constexpr bool UNROLL_Y = !FIXED || (ROOMY && MAT != JELLO);
     __shared__ RunShared<D> sm;
     extern __shared__ __align__(16) float4 recs[];
     unsigned short* runs = reinterpret_cast<unsigned short*>(recs + A.chunk_cap * run_rec4(D));
@@ -426,14 +435,19 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g_runs(ParticleBuf pb, cons
         unsigned err = 0;
         Stencil<D> st;
         if (make_stencil<D>(x, sc, st, err)) {
+            float F[D * D], aux;
+            if constexpr (PRELOAD) {
+#pragma unroll
+                for (int k = 0; k < D * D; ++k) F[k] = S[(Planes<D>::F + k) * cap + i];
+            }
             G2PAcc<D> acc;
-            g2p_window<D, PAGED, FIXED && !PAGED>(st, o, sm.tv, sc, A, acc);
+            g2p_window<D, PAGED, FIXED && !PAGED, UNROLL_Y>(st, o, sm.tv, sc, A, acc);
             // loaded after the gather, its register peak
             const GroupParams g = particle_group<FIXED>(A, pb, i);
-            float F[D * D], Cn[D * D], v[D], aux;
+            float Cn[D * D], v[D];
             typename SnowKeep<D>::T esvd;  // snow: the plasticity step's decomposition, reused by the stress
             err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux, MAT == SNOW ? &esvd : nullptr,
-                                            A.defer_vc != 0);
+                                            A.defer_vc != 0, PRELOAD);
             if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));
             Stencil<D> sn;
             if (make_stencil<D>(x, sc, sn, err)) {

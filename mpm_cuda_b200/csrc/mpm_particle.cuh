@@ -386,8 +386,9 @@ __device__ __forceinline__ void g2p_node(const Stencil<D>& st, const int* o, flo
 //       Sy = sum wx B10, Gy = sum wx B20, Sz = sum wx B01, Gz = sum wx B02
 // giving v = sum w v_i, S_b = sum w v_i o_b and G_b = h sum v_i dw/dx_b;
 // then B_ab = S_b[a] - fx_b v[a] (C = 4/h B) and grad v_ab = G_b[a] / h.
-// About half the multiply-adds of the node-by-node form.
-template <int D, class Fetch>
+// About half the multiply-adds of the node-by-node form.  UNROLL_Y: the y loop
+// unrolled too (3D), for callers with registers to spare.
+template <int D, bool UNROLL_Y = false, class Fetch>
 __device__ __forceinline__ void g2p_gather(const Stencil<D>& st, float inv_h, Fetch fetch, G2PAcc<D>& out) {
     float v[3] = {0.f, 0.f, 0.f}, S[3][3], G[3][3];
 #pragma unroll
@@ -416,10 +417,11 @@ __device__ __forceinline__ void g2p_gather(const Stencil<D>& st, float inv_h, Fe
 #pragma unroll 1
         for (int ox = 0; ox < 3; ++ox) {
             V3 B00 = zero(), B10 = zero(), B20 = zero(), B01 = zero(), B02 = zero();
-            // the y loop stays rolled: fully unrolled, the 27 hoisted tile
-            // loads and the partial sums exceed the register budget of the
-            // high-occupancy launch configurations and spill
-#pragma unroll 1
+            // the y loop stays rolled by default: fully unrolled, the 27 hoisted
+            // tile loads and the partial sums exceed the register budget of
+            // the high-occupancy launch configurations and spill
+            constexpr int kUnrollY = UNROLL_Y ? 3 : 1;
+#pragma unroll kUnrollY
             for (int oy = 0; oy < 3; ++oy) {
                 V3 A0 = zero(), A1 = zero(), A2 = zero();
 #pragma unroll
