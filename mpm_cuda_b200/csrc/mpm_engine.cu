@@ -2,10 +2,6 @@
 // launch sequences (binned fused path, unbinned path).
 #include "mpm_engine.cuh"
 
-#include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_select.cuh>
-#include <cub/iterator/counting_input_iterator.cuh>
-
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -39,9 +35,8 @@ enum {
     CNT_REBINS = 12,
     CNT_UPDATE_DONE = 13,
     CNT_POOL_FREE = 14,  // paged grid: height of the free stack
-    CNT_DET_BLOCKS = 15, // deterministic P2G: length of the ascending list of marked blocks
-    CNT_DET_RUNS = 16,   // deterministic P2G: number of runs of records sharing a base node
-    CNT_PLACED = 17,     // re-binning: particles given a segment so far
+    CNT_DET_RUNS = 15,   // deterministic P2G: number of runs of records sharing a base node
+    CNT_PLACED = 16,     // re-binning: particles given a segment so far
     CNT_N = 32
 };
 
@@ -392,10 +387,8 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
         msg = std::string("mpm_create: cudaMallocHost: ") + cudaGetErrorString(e);
         return MPM_ERR_NOMEM;
     }
-    for (int p = 0; p < 2; ++p) {
-        if ((rc = alloc((void**)&keys[p], cap * sizeof(unsigned long long), "sort keys")) != MPM_OK) return rc;
-        if ((rc = alloc((void**)&vals[p], cap * sizeof(unsigned), "sort values")) != MPM_OK) return rc;
-    }
+    if ((rc = alloc((void**)&keys, cap * sizeof(unsigned long long), "cell keys")) != MPM_OK) return rc;
+    if ((rc = alloc((void**)&ranks, cap * sizeof(unsigned), "cell ranks")) != MPM_OK) return rc;
     for (const GroupParams& g : groups_h) mat_present[g.type] = true;
     mat_slots = MatSlots{};
     for (int m = 0; m < kMats; ++m)
@@ -404,24 +397,9 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     // the binning's cell counters live at the physical block in a paged grid
     const long long n_cell_counts = grid_blocks_alloc() * 64 * mat_slots.n;
     if ((rc = alloc((void**)&cell_count, n_cell_counts * sizeof(int), "cell counts")) != MPM_OK) return rc;
-    // the deterministic path's buffers (it needs a dense grid)
-    if ((rc = alloc((void**)&cell_end, paged ? 16 : total_blocks * 64 * sizeof(int), "cell ends")) != MPM_OK)
+    if (deterministic() && (rc = alloc_det()) != MPM_OK) {
+        msg = "mpm_create: " + last_error;
         return rc;
-    {
-        const int src_planes = dim == 3 ? SrcPlanes<3>::COUNT : SrcPlanes<2>::COUNT;
-        if ((rc = alloc((void**)&det_src, paged ? 16 : (size_t)src_planes * cap * sizeof(float), "source records")) !=
-            MPM_OK)
-            return rc;
-        const int src_stride = dim == 3 ? SrcPlanes<3>::STRIDE : SrcPlanes<2>::STRIDE;
-        if ((rc = alloc((void**)&det_sorted, paged ? 16 : (size_t)src_stride * cap * sizeof(float),
-                        "sorted source records")) != MPM_OK)
-            return rc;
-        if ((rc = alloc((void**)&det_blocks, paged ? 16 : total_blocks * sizeof(int), "sorted block list")) != MPM_OK)
-            return rc;
-        if (deterministic() && (rc = alloc_det_partials()) != MPM_OK) {
-            msg = "mpm_create: " + last_error;
-            return rc;
-        }
     }
     if ((rc = alloc((void**)&seg_count, total_blocks * 4 * sizeof(int), "segment counts")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&seg_start, total_blocks * 4 * sizeof(int), "segment starts")) != MPM_OK) return rc;
@@ -435,23 +413,6 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     // partial chunk per non-empty block
     list_cap = cap / kMinChunkParticles + std::min<long long>(cap, total_blocks) + 1;
     if ((rc = alloc((void**)&chunks, kMats * list_cap * sizeof(Chunk), "chunks")) != MPM_OK) return rc;
-    // bits of the deterministic path's sort keys: node indices and the
-    // no-cell key (the node count) are all below 2^det_key_bits
-    det_key_bits = 1;
-    while (det_key_bits < 64 && (1LL << det_key_bits) <= total_blocks * 64) ++det_key_bits;
-    cub::DeviceRadixSort::SortPairs(nullptr, sort_tmp_bytes, keys[0], keys[1], vals[0], vals[1], (int)cap, 0, 64);
-    {
-        // the deterministic path's ascending list of marked blocks shares the temp space
-        size_t sel = 0;
-        cub::DeviceSelect::Flagged(nullptr, sel, cub::CountingInputIterator<int>(0), blk_flag, det_blocks,
-                                   counters + CNT_DET_BLOCKS, (int)total_blocks);
-        sort_tmp_bytes = std::max(sort_tmp_bytes, sel);
-        // and the list of runs of sorted records
-        cub::DeviceSelect::If(nullptr, sel, cub::CountingInputIterator<int>(0), det_runs, counters + CNT_DET_RUNS,
-                              (int)cap, RunStart{keys[1], det_no_cell()});
-        sort_tmp_bytes = std::max(sort_tmp_bytes, sel);
-    }
-    if ((rc = alloc(&sort_tmp, sort_tmp_bytes, "sort temp")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&pos_out, cap * D * sizeof(float), "positions")) != MPM_OK) return rc;
 
     e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
@@ -471,7 +432,6 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     if (e == cudaSuccess) e = cudaMemset(err_d, 0, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(blk_flag, 0, total_blocks * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(cell_count, 0, n_cell_counts * sizeof(int));
-    if (e == cudaSuccess && !paged) e = cudaMemset(cell_end, 0, total_blocks * 64 * sizeof(int));
     if (e == cudaSuccess && paged) {
         k_fill_int<<<grid_blocks(total_blocks, 256), 256>>>(pages.page, total_blocks, pages.trash);
         k_fill_stack<<<grid_blocks(pool_cap, 256), 256>>>(pages.free_slots, pool_cap);
@@ -751,9 +711,9 @@ void Engine::release() {
         gp[p] = nullptr;
         ids[p] = nullptr;
     }
-    void* ptrs[] = {groups_d, scenes_d, grid_mom, grid_vel, err_d, keys[0], keys[1], vals[0], vals[1],
-                    cell_count, seg_count, seg_start, sort_tmp, blk_flag, active, blk_epoch, counters, chunks,
-                    pos_out, cell_end, det_src, det_sorted, det_blocks, det_runs, det_partial,
+    void* ptrs[] = {groups_d, scenes_d, grid_mom, grid_vel, err_d, keys, ranks,
+                    cell_count, seg_count, seg_start, blk_flag, active, blk_epoch, counters, chunks,
+                    pos_out, det_cells, det_rows, det_slots, det_order, det_runs, det_partial,
                     sur_counts, speed_max, scene_time,
                     pages.page, pages.slot_block, pages.free_slots};
     for (void* p : ptrs) cudaFree(p);
@@ -764,13 +724,13 @@ void Engine::release() {
     scenes_d = nullptr;
     grid_mom = grid_vel = nullptr;
     err_d = nullptr;
-    keys[0] = keys[1] = nullptr;
-    vals[0] = vals[1] = nullptr;
-    cell_count = seg_count = seg_start = cell_end = nullptr;
-    det_src = det_sorted = nullptr;
-    det_blocks = det_runs = nullptr;
-    det_partial = nullptr;
-    sort_tmp = nullptr;
+    keys = nullptr;
+    ranks = nullptr;
+    cell_count = seg_count = seg_start = nullptr;
+    det_cells = nullptr;
+    det_runs = nullptr;
+    det_rows = det_partial = nullptr;
+    det_slots = det_order = nullptr;
     blk_flag = nullptr;
     active = blk_epoch = counters = nullptr;
     chunks = nullptr;
@@ -857,7 +817,7 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
     // next one rewrites, stay behind
     const bool reclaim = in_loop;
     const int to = 1 - from;
-    int* rank = reinterpret_cast<int*>(vals[0]);
+    int* rank = reinterpret_cast<int*>(ranks);
     if (paged && reclaim) {
         // blocks with nothing active near them give their physical block back
         auto k = dim == 3 ? k_pool_reclaim<3> : k_pool_reclaim<2>;
@@ -884,7 +844,7 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
                                    : (cm ? k_bin_count<2, false, true> : k_bin_count<2, false, false>));
         note_launch_status("k_bin_count",
                            cudaLaunchKernelEx(&lc, k, buf(from), n_particles, (const GroupParams*)groups_d,
-                                              (const SceneParams*)scenes_d, mat_slots, keys[0], rank, cell_count,
+                                              (const SceneParams*)scenes_d, mat_slots, keys, rank, cell_count,
                                               seg_count, pages, bc));
     }
     lc.gridDim = dim3(grid_blocks(total_blocks, 256));
@@ -900,7 +860,7 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
                           : (paged ? (cm ? k_bin_place<2, true, true> : k_bin_place<2, true, false>)
                                    : (cm ? k_bin_place<2, false, true> : k_bin_place<2, false, false>));
         note_launch_status("k_bin_place",
-                           cudaLaunchKernelEx(&lc, k, buf(from), buf(to), n_particles, (const unsigned long long*)keys[0],
+                           cudaLaunchKernelEx(&lc, k, buf(from), buf(to), n_particles, (const unsigned long long*)keys,
                                               (const int*)rank, (const int*)cell_count, (const int*)seg_count,
                                               (const int*)seg_start, mat_slots, in_loop ? 0 : 1, err_d, pages));
     }
@@ -1032,86 +992,60 @@ void Engine::enqueue_adapt_dt() {
     note_launch_status("k_adapt_dt", cudaLaunchKernelEx(&lc, k_adapt_dt, scenes_d, n_scenes, speed_max, scene_time));
 }
 
-// deterministic P2G of the current state into grid_mom (blocks marked active)
-void Engine::enqueue_det_p2g() {
+// Deterministic P2G of the current state into grid_mom (step = false; blocks
+// marked active), or G2P and update from the velocities of the last grid update
+// and then the P2G of the result
+template <int D>
+void Engine::enqueue_det(bool step) {
     const int n_scenes = (int)scenes_h.size();
+    const DetCells dc{det_cells, keys, (unsigned long long)total_blocks * 64, ranks};
+    const DetCounters cnt{counters + CNT_DET_RUNS, counters + CNT_PLACED};
+    const int* n_active = counters + CNT_ACTIVE;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t lc = pdl_config(update_ctas, 256, 0, stream, &attr);
     if (n_particles > 0) {
-        if (dim == 3)
-            k_det_source<3><<<grid_blocks(n_particles, 128), 128, 0, stream>>>(
-                buf(cur), n_particles, groups_d, scenes_d, det_src, cap, keys[0], det_no_cell(), vals[0], blk_flag,
-                active, counters + CNT_ACTIVE, err_d);
+        const unsigned nb = grid_blocks(n_particles, 128);
+        if (step)
+            k_det_step<D><<<nb, 128, 0, stream>>>(buf(cur), n_particles, groups_d, scenes_d, grid_vel, det_rows, dc,
+                                                  blk_flag, active, counters + CNT_ACTIVE, cnt, counters + CNT_EPOCH,
+                                                  err_d);
         else
-            k_det_source<2><<<grid_blocks(n_particles, 128), 128, 0, stream>>>(
-                buf(cur), n_particles, groups_d, scenes_d, det_src, cap, keys[0], det_no_cell(), vals[0], blk_flag,
-                active, counters + CNT_ACTIVE, err_d);
+            k_det_source<D><<<nb, 128, 0, stream>>>(buf(cur), n_particles, groups_d, scenes_d, det_rows, dc, blk_flag,
+                                                    active, counters + CNT_ACTIVE, cnt, err_d);
         note_launch("k_det_source");
-        // keys are node indices below the no-cell key (the node count), which
-        // sorts last: the sort needs only the bits that hold the node count
-        cub::DeviceRadixSort::SortPairs(sort_tmp, sort_tmp_bytes, keys[0], keys[1], vals[0], vals[1],
-                                        (int)n_particles, 0, det_key_bits, stream);
-        note_launch("cub::DeviceRadixSort::SortPairs");
-        k_det_ranges<<<grid_blocks(n_particles, 256), 256, 0, stream>>>(keys[1], n_particles, det_no_cell(),
-                                                                        cell_count, cell_end);
-        note_launch("k_det_ranges");
-        if (dim == 3)
-            k_det_permute<3><<<grid_blocks(n_particles, 256), 256, 0, stream>>>(det_src, (float4*)det_sorted, cap,
-                                                                                vals[1], n_particles);
-        else
-            k_det_permute<2><<<grid_blocks(n_particles, 256), 256, 0, stream>>>(det_src, (float4*)det_sorted, cap,
-                                                                                vals[1], n_particles);
-        note_launch("k_det_permute");
+        note_launch_status("k_det_starts", cudaLaunchKernelEx(&lc, k_det_starts, det_cells, (const int*)active, n_active,
+                                                              det_runs, cnt));
+        lc.gridDim = dim3(grid_blocks(n_particles, 256));
+        note_launch_status("k_det_slots", cudaLaunchKernelEx(&lc, k_det_slots, dc, n_particles, det_slots));
+        note_launch_status("k_det_order", cudaLaunchKernelEx(&lc, k_det_order, dc, n_particles, (const unsigned*)det_slots,
+                                                             (const int*)cnt.placed, det_order));
+        lc.gridDim = dim3(num_sms * 8);
+        lc.blockDim = dim3(64);
+        note_launch_status("k_det_partials",
+                           cudaLaunchKernelEx(&lc, k_det_partials<D>, (const float4*)det_rows,
+                                              (const unsigned*)det_order, (const int4*)det_runs, (const int*)cnt.n_runs,
+                                              (const SceneParams*)scenes_d, n_scenes, det_partial));
+    } else if (step) {
+        k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_EPOCH);
+        note_launch("epoch");
     }
-    if (n_particles > 0) {
-        // the runs of records sharing a base node, and their partial sums
-        cub::DeviceSelect::If(sort_tmp, sort_tmp_bytes, cub::CountingInputIterator<int>(0), det_runs,
-                              counters + CNT_DET_RUNS, (int)n_particles, RunStart{keys[1], det_no_cell()}, stream);
-        note_launch("cub::DeviceSelect::If");
-        if (dim == 3)
-            k_det_partials<3><<<num_sms * 8, 64, 0, stream>>>((const float4*)det_sorted, keys[1], det_runs,
-                                                              counters + CNT_DET_RUNS, cell_end, scenes_d, n_scenes,
-                                                              det_partial);
-        else
-            k_det_partials<2><<<num_sms * 8, 64, 0, stream>>>((const float4*)det_sorted, keys[1], det_runs,
-                                                              counters + CNT_DET_RUNS, cell_end, scenes_d, n_scenes,
-                                                              det_partial);
-        note_launch("k_det_partials");
-    }
-    // the blocks the source records marked, in ascending order
-    cub::DeviceSelect::Flagged(sort_tmp, sort_tmp_bytes, cub::CountingInputIterator<int>(0), blk_flag, det_blocks,
-                               counters + CNT_DET_BLOCKS, (int)total_blocks, stream);
-    note_launch("cub::DeviceSelect::Flagged");
-    if (dim == 3)
-        k_det_sum<3><<<update_ctas, 256, 0, stream>>>(det_partial, cell_count, cell_end, det_blocks,
-                                                      counters + CNT_DET_BLOCKS, scenes_d, n_scenes, grid_mom);
-    else
-        k_det_sum<2><<<update_ctas, 256, 0, stream>>>(det_partial, cell_count, cell_end, det_blocks,
-                                                      counters + CNT_DET_BLOCKS, scenes_d, n_scenes, grid_mom);
-    note_launch("k_det_sum");
-    if (n_particles > 0) {
-        k_det_reset<<<grid_blocks(n_particles, 256), 256, 0, stream>>>(keys[1], n_particles, det_no_cell(),
-                                                                       cell_count, cell_end);
-        note_launch("k_det_reset");
-    }
+    lc.gridDim = dim3(update_ctas);
+    lc.blockDim = dim3(256);
+    note_launch_status("k_det_sum", cudaLaunchKernelEx(&lc, k_det_sum<D>, (const float4*)det_partial,
+                                                       (const int2*)det_cells, (const int*)active, n_active,
+                                                       (const SceneParams*)scenes_d, n_scenes, grid_mom));
+    note_launch_status("k_det_reset", cudaLaunchKernelEx(&lc, k_det_reset, det_cells, (const int*)active, n_active));
+}
+
+void Engine::enqueue_det_p2g(bool step) {
+    if (dim == 3) enqueue_det<3>(step);
+    else enqueue_det<2>(step);
 }
 
 // grid update of the pending P2G, G2P from it, deterministic P2G of the result
 void Engine::enqueue_det_substep() {
     enqueue_grid_update();
-    const ParticleBuf pb = buf(cur);
-    const int bt = opt.block_threads > 0 ? opt.block_threads : 128;
-    if (n_particles > 0) {
-        if (dim == 3)
-            k_g2p_direct<3><<<grid_blocks(n_particles, bt), bt, 0, stream>>>(pb, n_particles, groups_d, scenes_d,
-                                                                             grid_vel, err_d);
-        else
-            k_g2p_direct<2><<<grid_blocks(n_particles, bt), bt, 0, stream>>>(pb, n_particles, groups_d, scenes_d,
-                                                                             grid_vel, err_d);
-        note_launch("k_g2p_direct");
-    }
-    // the epoch is bumped once per substep (the fused kernel does it in its path)
-    k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_EPOCH);
-    note_launch("epoch");
-    enqueue_det_p2g();
+    enqueue_det_p2g(true);
 }
 
 // moves the particles back to creation order (deterministic mode needs an
@@ -1171,7 +1105,7 @@ int Engine::prologue() {
     if (deterministic()) {
         int rc = canonical_order();
         if (rc != MPM_OK) return rc;
-        enqueue_det_p2g();
+        enqueue_det_p2g(false);
         rc = take_launch_error();
         if (rc != MPM_OK) return rc;
         grid_dirty = false;
@@ -1622,17 +1556,29 @@ int Engine::bin_stats(int64_t* fallbacks, int64_t* rebins) {
     return MPM_OK;
 }
 
-// The deterministic path's partial sums (3^D float4 per particle slot) and run
-// list, allocated when the path is first chosen
-int Engine::alloc_det_partials() {
+// The deterministic path's buffers (source records, cells, order and run list,
+// 3^D float4 of partial sums per particle slot), allocated when the path is first
+// chosen
+int Engine::alloc_det() {
     if (det_partial) return MPM_OK;
-    const int k = dim == 3 ? 27 : 9;
-    if (cudaMalloc((void**)&det_partial, (size_t)cap * k * sizeof(float4)) != cudaSuccess ||
-        cudaMalloc((void**)&det_runs, (size_t)cap * sizeof(int)) != cudaSuccess) {
+    const size_t k = dim == 3 ? 27 : 9, row = dim == 3 ? SrcRow<3>::N4 : SrcRow<2>::N4;
+    const size_t nodes = (size_t)total_blocks * 64;
+    struct {
+        void** p;
+        size_t bytes;
+    } const want[] = {{(void**)&det_cells, nodes * sizeof(int2)},      {(void**)&det_rows, cap * row * sizeof(float4)},
+                      {(void**)&det_slots, cap * sizeof(unsigned)},    {(void**)&det_order, cap * sizeof(unsigned)},
+                      {(void**)&det_runs, cap * sizeof(int4)},         {(void**)&det_partial, cap * k * sizeof(float4)}};
+    bool ok = true;
+    for (const auto& w : want) ok = ok && cudaMalloc(w.p, w.bytes) == cudaSuccess;
+    ok = ok && cudaMemset(det_cells, 0, nodes * sizeof(int2)) == cudaSuccess;
+    if (!ok) {
         cudaGetLastError();
-        cudaFree(det_partial);
-        det_partial = nullptr;
-        last_error = "mpm: out of device memory for the deterministic path's partial sums";
+        for (const auto& w : want) {
+            cudaFree(*w.p);
+            *w.p = nullptr;
+        }
+        last_error = "mpm: out of device memory for the deterministic path's buffers";
         return MPM_ERR_NOMEM;
     }
     return MPM_OK;
@@ -1658,7 +1604,7 @@ int Engine::set_p2g_mode(int mode) {
     }
     MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
     if (mode == MPM_P2G_DETERMINISTIC) {
-        const int rc = alloc_det_partials();
+        const int rc = alloc_det();
         if (rc != MPM_OK) return rc;
     }
     opt.p2g_mode = mode;
@@ -1807,7 +1753,7 @@ int Engine::profile_stages(int n, float* out_ms, int n_out, int* n_written) {
             note_launch("k_g2p_direct");
             k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_EPOCH);
             cudaEventRecord(ev[2], stream);
-            enqueue_det_p2g();
+            enqueue_det_p2g(false);
             cudaEventRecord(ev[3], stream);
             cudaEventSynchronize(ev[3]);
             for (int st_i = 0; st_i < 3; ++st_i) {

@@ -48,28 +48,26 @@ struct Engine {
     unsigned* err_h = nullptr;  // page-locked copy of the error word
 
     // binning and block activity
-    // binning: keys[0] = (home block, material, cell) and vals[0] = rank in
-    // the cell of each particle; the deterministic mode sorts keys / vals
-    unsigned long long* keys[2] = {nullptr, nullptr};
-    unsigned* vals[2] = {nullptr, nullptr};
-    // binning: per (block, present material) 64 cell counts; the
-    // deterministic mode: per base node of every block
+    // binning: (home block, material, cell) and rank in the cell of each particle;
+    // deterministic mode: base node and arrival number at it
+    unsigned long long* keys = nullptr;
+    unsigned* ranks = nullptr;
+    // binning: per (block, present material) 64 cell counts
     int* cell_count = nullptr;
     MatSlots mat_slots{};       // compact index of each present material
-    int* cell_end = nullptr;    // deterministic mode: end of each base node's records
-    float* det_src = nullptr;   // deterministic mode: P2G source records
-    float* det_sorted = nullptr;  // the same records in sorted order
-    int* det_blocks = nullptr;    // the blocks they mark, ascending
-    int* det_runs = nullptr;      // first sorted position of each run sharing a base node
-    float4* det_partial = nullptr;  // per (run, stencil offset) partial sums (allocated on first use)
-    int det_key_bits = 64;
-    // sort key of a particle whose stencil left the grid: one past the last node
-    unsigned long long det_no_cell() const { return (unsigned long long)total_blocks * 64; }
+    // deterministic mode (allocated on first use): per base node of every block
+    // its run, P2G source records in creation order, particles by run in arrival
+    // and in creation order, (block, first place, end) of each run, per (run, stencil
+    // offset) partial sums
+    int2* det_cells = nullptr;
+    float4* det_rows = nullptr;
+    unsigned* det_slots = nullptr;
+    unsigned* det_order = nullptr;
+    int4* det_runs = nullptr;
+    float4* det_partial = nullptr;
     bool sorted_order = false;  // particles permuted away from creation order
     int* seg_count = nullptr;   // per (block, material)
     int* seg_start = nullptr;
-    void* sort_tmp = nullptr;
-    size_t sort_tmp_bytes = 0;
     Chunk* chunks = nullptr;    // kMats lists of list_cap entries
     long long list_cap = 0;
     bool mat_present[3] = {false, false, false};
@@ -152,7 +150,7 @@ struct Engine {
     int get_grid(int scene, float* mass, float* vel);
     int count_active_nodes(int scene, int64_t* n);
     int set_p2g_mode(int mode);
-    int alloc_det_partials();
+    int alloc_det();
     int set_stress_mode(int mode, Surrogate* s);
     int stress_stats(int64_t* net, int64_t* fallback);
     int scene_time_of(int scene, double* t, float* dt);
@@ -192,7 +190,9 @@ struct Engine {
     void sur_occupancy();
     int sur_chunk() const;
     int sur_refresh();
-    void enqueue_det_p2g();
+    void enqueue_det_p2g(bool step);
+    template <int D>
+    void enqueue_det(bool step);
     void enqueue_det_substep();
     int canonical_order();
 };

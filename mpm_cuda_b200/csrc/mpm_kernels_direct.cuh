@@ -77,39 +77,29 @@ __global__ void __launch_bounds__(256) k_grid_update_dense(float4* __restrict__ 
     if (clear_src) mom[gi] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// G2P + F update + advection straight from global memory
-// (InterpolateAndMove, MPMCUDA.cu:474-741).
+// G2P + F update + advection of particle i straight from global memory
+// (InterpolateAndMove, MPMCUDA.cu:474-741), its new state stored and returned;
+// false when the stencil left the grid (nothing changes).  F is neither read nor
+// stored for water.
 template <int D>
-__global__ void __launch_bounds__(128) k_g2p_direct(ParticleBuf pb, long long n,
-                                                    const GroupParams* __restrict__ groups,
-                                                    const SceneParams* __restrict__ scenes,
-                                                    const float4* __restrict__ grid, unsigned* err_word) {
+__device__ __forceinline__ bool g2p_update(const ParticleBuf& pb, long long i, const GroupParams& g,
+                                           const SceneParams& sc, const float4* __restrict__ grid, float* x, float* v,
+                                           float* C, float* F, float& aux, unsigned& err) {
     using P = Planes<D>;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     float* s = pb.s;
     const long long cap = pb.cap;
-    float x[D];
 #pragma unroll
     for (int a = 0; a < D; ++a) x[a] = s[(P::X + a) * cap + i];
-    const GroupParams g = groups[pb.grp[i]];
-    const SceneParams& sc = scenes[g.scene];
-    unsigned err = 0;
     Stencil<D> st;
-    if (!make_stencil<D>(x, sc, st, err)) {
-        atomicOr(err_word, err);
-        return;
-    }
+    if (!make_stencil<D>(x, sc, st, err)) return false;
     G2PAcc<D> acc;
     const float inv_h = sc.inv_h;
     const StencilIndex<D> ix(sc, st.base);
     const float4* gs = grid + sc.node_off;
     g2p_gather<D>(st, inv_h, [&](int ox, int oy, int oz) { return __ldg(&gs[ix(ox, oy, D == 3 ? oz : 0)]); }, acc);
-    float F[D * D], aux = s[P::AUX * cap + i];
-    if (g.type != WATER) {
+    aux = s[P::AUX * cap + i];
 #pragma unroll
-        for (int k = 0; k < D * D; ++k) F[k] = s[(P::F + k) * cap + i];
-    }
+    for (int k = 0; k < D * D; ++k) F[k] = g.type != WATER ? s[(P::F + k) * cap + i] : 0.f;
     err |= material_update<D>(acc, sc.dt, g, F, aux);
     if (g.type != WATER) {
 #pragma unroll
@@ -119,13 +109,31 @@ __global__ void __launch_bounds__(128) k_g2p_direct(ParticleBuf pb, long long n,
     const float c4 = 4.f * inv_h;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-        const float xn = fmaf(sc.dt, acc.v[a], x[a]);
-        if (!isfinite(xn)) err |= ERR_NONFINITE;
-        s[(P::X + a) * cap + i] = xn;
-        s[(P::V + a) * cap + i] = acc.v[a];
+        x[a] = fmaf(sc.dt, acc.v[a], x[a]);
+        v[a] = acc.v[a];
+        if (!isfinite(x[a])) err |= ERR_NONFINITE;
+        s[(P::X + a) * cap + i] = x[a];
+        s[(P::V + a) * cap + i] = v[a];
 #pragma unroll
-        for (int b = 0; b < D; ++b) s[(P::C + a * D + b) * cap + i] = c4 * acc.B[a * D + b];
+        for (int b = 0; b < D; ++b) {
+            C[a * D + b] = c4 * acc.B[a * D + b];
+            s[(P::C + a * D + b) * cap + i] = C[a * D + b];
+        }
     }
+    return true;
+}
+
+template <int D>
+__global__ void __launch_bounds__(128) k_g2p_direct(ParticleBuf pb, long long n,
+                                                    const GroupParams* __restrict__ groups,
+                                                    const SceneParams* __restrict__ scenes,
+                                                    const float4* __restrict__ grid, unsigned* err_word) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const GroupParams g = groups[pb.grp[i]];
+    float x[D], v[D], C[D * D], F[D * D], aux;
+    unsigned err = 0;
+    g2p_update<D>(pb, i, g, scenes[g.scene], grid, x, v, C, F, aux, err);
     if (err) atomicOr(err_word, err);
 }
 
