@@ -1004,14 +1004,14 @@ void Engine::enqueue_det(bool step) {
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t lc = pdl_config(update_ctas, 256, 0, stream, &attr);
     if (n_particles > 0) {
-        const unsigned nb = grid_blocks(n_particles, 128);
         if (step)
-            k_det_step<D><<<nb, 128, 0, stream>>>(buf(cur), n_particles, groups_d, scenes_d, grid_vel, det_rows, dc,
-                                                  blk_flag, active, counters + CNT_ACTIVE, cnt, counters + CNT_EPOCH,
-                                                  err_d);
+            k_det_step<D><<<grid_blocks(n_particles, kDetStepThreads), kDetStepThreads, 0, stream>>>(
+                buf(cur), n_particles, groups_d, scenes_d, grid_vel, det_rows, dc, blk_flag, active,
+                counters + CNT_ACTIVE, cnt, counters + CNT_EPOCH, err_d);
         else
-            k_det_source<D><<<nb, 128, 0, stream>>>(buf(cur), n_particles, groups_d, scenes_d, det_rows, dc, blk_flag,
-                                                    active, counters + CNT_ACTIVE, cnt, err_d);
+            k_det_source<D><<<grid_blocks(n_particles, 128), 128, 0, stream>>>(
+                buf(cur), n_particles, groups_d, scenes_d, det_rows, dc, blk_flag, active, counters + CNT_ACTIVE, cnt,
+                err_d);
         note_launch("k_det_source");
         note_launch_status("k_det_starts", cudaLaunchKernelEx(&lc, k_det_starts, det_cells, (const int*)active, n_active,
                                                               det_runs, cnt));

@@ -20,11 +20,9 @@
 // by bytes.  A radix sort of 238k keys runs 27 CTAs, three passes of 13 us; the
 // counting sort's three kernels take 13 us together, and G2P, update and source of
 // a particle are one kernel.  Jello cube of 238k particles in a 101^3 grid: the
-// substep takes 109 us instead of 171 (2.1M particles in 256^3: 530 instead of
-// 712), bit for bit the radix sort's result.  Of that (cold caches, one launch
-// at a time) 48 us are k_det_step, 26 k_det_partials, 25 k_det_sum, 5 the grid
-// update.  Three threads per run, one per x-plane, were slower (35 us for the
-// partials) and round differently.
+// substep takes 86 us instead of 171 (2.1M particles in 256^3: 474 instead of
+// 712), bit for bit the radix sort's result.  Three threads per run, one per
+// x-plane, were slower (35 us against 26 for the partials) and round differently.
 #pragma once
 
 #include "mpm_grid.cuh"
@@ -117,9 +115,12 @@ __global__ void __launch_bounds__(128) k_det_source(ParticleBuf pb, long long n,
 }
 
 // G2P, update and the next substep's source record of every particle
-// (k_g2p_direct and k_det_source in one pass over the state); the epoch moves on
+// (k_g2p_direct and k_det_source in one pass over the state); the epoch moves on.
+// Ten CTAs of 64 threads an SM hold 20 warps at 96 registers; left alone, the
+// compiler takes 124 (16 warps): the substep 98 us against 93.
+constexpr int kDetStepThreads = 64;
 template <int D>
-__global__ void __launch_bounds__(128) k_det_step(ParticleBuf pb, long long n, const GroupParams* __restrict__ groups,
+__global__ void __launch_bounds__(kDetStepThreads, 10) k_det_step(ParticleBuf pb, long long n, const GroupParams* __restrict__ groups,
                                                   const SceneParams* __restrict__ scenes,
                                                   const float4* __restrict__ grid, float4* __restrict__ rows,
                                                   DetCells dc, unsigned* __restrict__ blk_flag,
@@ -233,16 +234,24 @@ __global__ void __launch_bounds__(64, 4) k_det_partials(const float4* __restrict
         float4 acc[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // the next record is on its way while this one is summed
+        float4 nxt[SR::N4];
+        unsigned next = j0 + 1 < j1 ? order[j0 + 1] : 0;
+#pragma unroll
+        for (int q = 0; q < SR::N4; ++q) nxt[q] = rows[(long long)order[j0] * SR::N4 + q];
         for (int j = j0; j < j1; ++j) {
-            const float4* row = rows + (long long)order[j] * SR::N4;
             float rec[SR::N4 * 4];
 #pragma unroll
             for (int q = 0; q < SR::N4; ++q) {
-                const float4 v = row[q];
-                rec[4 * q] = v.x;
-                rec[4 * q + 1] = v.y;
-                rec[4 * q + 2] = v.z;
-                rec[4 * q + 3] = v.w;
+                rec[4 * q] = nxt[q].x;
+                rec[4 * q + 1] = nxt[q].y;
+                rec[4 * q + 2] = nxt[q].z;
+                rec[4 * q + 3] = nxt[q].w;
+            }
+            if (j + 1 < j1) {
+#pragma unroll
+                for (int q = 0; q < SR::N4; ++q) nxt[q] = rows[(long long)next * SR::N4 + q];
+                if (j + 2 < j1) next = order[j + 2];
             }
             Stencil<D> st;
             P2GSource<D> s;
@@ -281,9 +290,11 @@ __global__ void __launch_bounds__(256) k_det_reset(int2* __restrict__ cells, con
 
 // Every node of the listed blocks adds, in the order of the stencil offset o,
 // the partial sums of the base nodes node - o, o in {0,1,2}^D, and stores the
-// total.
+// total.  Nine loads in flight instead of one: the substep of 109 us takes 100,
+// and 3 CTAs an SM, so that they stay in registers, 91 (with 64-thread
+// k_det_step CTAs and the next record ahead in k_det_partials).
 template <int D>
-__global__ void __launch_bounds__(256) k_det_sum(const float4* __restrict__ partial,
+__global__ void __launch_bounds__(256, 3) k_det_sum(const float4* __restrict__ partial,
                                                  const int2* __restrict__ cells, const int* __restrict__ blocks,
                                                  const int* __restrict__ n_blocks,
                                                  const SceneParams* __restrict__ scenes, int n_scenes,
@@ -302,22 +313,29 @@ __global__ void __launch_bounds__(256) k_det_sum(const float4* __restrict__ part
         const bool in_grid = id[0] < sc.n[0] && id[1] < sc.n[1] && (D == 2 || id[2] < sc.n[2]);
         if (in_grid) {
 #pragma unroll
-            for (int ox = 0; ox < 3; ++ox)
+            for (int ox = 0; ox < 3; ++ox) {
+                constexpr int P = D == 3 ? 9 : 3;
+                // the runs of an x-plane of base nodes, then their partial sums: loads that do not wait on one another
+                int j[P];
 #pragma unroll
-                for (int oy = 0; oy < 3; ++oy)
+                for (int q = 0; q < P; ++q) {
+                    const int bx = id[0] - ox, by = id[1] - (D == 3 ? q / 3 : q), bz = D == 3 ? id[2] - q % 3 : 0;
+                    const int2 run = bx < 0 || by < 0 || bz < 0 ? make_int2(0, 0) : cells[node_index<D>(sc, bx, by, bz)];
+                    j[q] = run.y > run.x ? run.x : -1;  // -1: no particle has this base node
+                }
+                float4 c[P];
 #pragma unroll
-                    for (int oz = 0; oz < (D == 3 ? 3 : 1); ++oz) {
-                        const int bx = id[0] - ox, by = id[1] - oy, bz = D == 3 ? id[2] - oz : 0;
-                        if (bx < 0 || by < 0 || bz < 0) continue;
-                        const long long cell = node_index<D>(sc, bx, by, bz);
-                        const int2 j = cells[cell];
-                        if (j.y <= j.x) continue;  // no particle has this base node
-                        const float4 c = partial[(long long)j.x * K + (D == 3 ? (ox * 3 + oy) * 3 + oz : ox * 3 + oy)];
-                        acc.x += c.x;
-                        acc.y += c.y;
-                        acc.z += c.z;
-                        acc.w += c.w;
-                    }
+                for (int q = 0; q < P; ++q)
+                    c[q] = j[q] < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : partial[(long long)j[q] * K + ox * P + q];
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    if (j[q] < 0) continue;
+                    acc.x += c[q].x;
+                    acc.y += c[q].y;
+                    acc.z += c[q].z;
+                    acc.w += c[q].w;
+                }
+            }
         }
         grid_mom[(long long)b * 64 + lane] = acc;
     }
