@@ -900,7 +900,7 @@ int Engine::encode_vel_map() {
     return r == CUDA_SUCCESS ? MPM_OK : MPM_ERR_UNSUPPORTED;
 }
 
-FusedArgs Engine::fused_args(int mat, bool bump) {
+FusedArgs Engine::fused_args(int mat, bool first) {
     FusedArgs A;
     A.chunks = chunks + mat * list_cap;
     A.n_chunks = counters + CNT_CHUNKS + mat;
@@ -915,7 +915,7 @@ FusedArgs Engine::fused_args(int mat, bool bump) {
     A.active = active;
     A.n_active = counters + CNT_ACTIVE;
     A.epoch = counters + CNT_EPOCH;
-    A.bump_epoch = bump ? 1 : 0;
+    A.first = first ? 1 : 0;
     A.err_word = err_d;
     A.fallback = (unsigned*)(counters + CNT_FALLBACK);
     A.speed_max = opt.adaptive_dt ? speed_max : nullptr;
@@ -955,11 +955,11 @@ void Engine::enqueue_grid_update() {
 }
 
 void Engine::enqueue_g2p2g(int parity) {
-    bool bump = true;
+    bool first = true;
     for (int mat = 0; mat < kMats; ++mat) {
         if (!mat_present[mat]) continue;
-        const FusedArgs A = fused_args(mat, bump);
-        bump = false;
+        const FusedArgs A = fused_args(mat, first);
+        first = false;
         if (sur_kernel(mat)) {
             const SurArgs SA{&sur->weights->f, sur->meta, sur_counts};
             const int ch = sur_chunk();

@@ -178,7 +178,7 @@ struct Engine {
     void enqueue_grid_update();
     void enqueue_adapt_dt();
     void enqueue_g2p2g(int parity);
-    FusedArgs fused_args(int mat, bool bump);
+    FusedArgs fused_args(int mat, bool first);
     int prologue();
     int build_graph(int parity, int rebin, int count, cudaGraphExec_t* out);
     void drop_graphs();

@@ -259,18 +259,16 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
     }
     // The chunk list and the particles were last written before the grid update
     // ahead of this launch began: a CTA starts once that kernel's CTAs (or those
-    // of another material's pass, which wait for it) have all passed their own
-    // wait.  So the first chunk's record and positions are fetched before this
-    // kernel's wait; velocities, cursors and block flags after it.
+    // of another material's pass) have all passed their own wait.  So the first
+    // chunk's record and positions are fetched before this kernel's wait;
+    // velocities, cursors and block flags after it.
     const ChunkList list(A);
     const int nch = list.all;
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
     if (threadIdx.x == 0 && cur < nch) sm.ch[0] = *list.at(A, cur);
     __syncthreads();  // the record, the barrier and the lists initialised
-    pdl_wait();     // the grid update ahead of this launch has finished
-    pdl_trigger();  // the next pass may launch; it waits for this one to end
-    if (A.bump_epoch && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.epoch, 1);
+    pass_begin(A);    // the grid update ahead has finished
     if (cur < nch) load_window<D, CHUNK, FIXED, PAGED>(A, sm.ch[0], sm.tv, sm.s27[0], &sm.bar);
     cp_async_commit();
     SpeedFlush speed;
@@ -409,6 +407,7 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
         cur = next_chunk;
     }
     speed.flush(A.speed_max);
+    pass_end(A);
 }
 
 template <int D, int MAT, int CHUNK, int MINB, bool FIXED, bool PAGED>
