@@ -400,7 +400,8 @@ def run_ours(args, rank, world, local_rank, dist):
     if args.mode == "binned":
         # the two other ceilings of the fused kernel, beside HBM: its FP32 rate
         # against the SMs' non-tensor FP32 peak at the sampled clock, and its
-        # node reductions (27 per particle in 3D, 9 in 2D)
+        # node contributions (27 per particle in 3D, 9 in 2D; a configuration
+        # with run sums adds the particles of a base node before it reduces)
         fused_s = stages[stage_names.index("g2p2g")] * 1e-3
         props = torch.cuda.get_device_properties(local_rank)
         mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 0.0
@@ -416,7 +417,7 @@ def run_ours(args, rank, world, local_rank, dist):
                                           "peak = SMs x 128 FP32 lanes x 2 x median SM clock"}
         per = 27 if scenes[0].dim == 3 else 9
         roofline["reductions"] = {"per_particle": per, "achieved": round(per * n_part / fused_s / 1e9, 1),
-                                  "unit": "G node reductions/s (red.global.add.v4.f32)",
+                                  "unit": "G node contributions/s (reduced by red.global.add.v4.f32)",
                                   "l2_requests_per_particle": measured_counter(args.workload, "g2p2g",
                                                                                "l2_red_requests_per_particle")}
 
@@ -478,7 +479,7 @@ def run_ours(args, rank, world, local_rank, dist):
             "warmup": args.warmup, "ms_per_step": t_max_s * 1e3 / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded)",
             "config": {"workload": desc, "particles_per_gpu": n_part, "particles_total": int(total_particles),
-                       "active_nodes": active_nodes, "stress": "plain (SVD)", "path": args.mode,
+                       "active_nodes": active_nodes, "stress": "plain", "path": args.mode,
                        "tile_fallbacks": fallbacks, "rebins": rebins,
                        "grid": grid_desc,
                        "kernel_config": {"index": kcfg, "chunk": chunk.value, "min_ctas_per_sm": min_ctas.value,
@@ -487,8 +488,8 @@ def run_ours(args, rank, world, local_rank, dist):
                        "l2": l2_desc,
                        "parallelism": f"replicas x{world}" if args.workload != "c4" else f"scenes split over {world}"},
             "roofline": roofline, "e2e": e2e, "surrogate": sur,
-            # 7 kernels per re-binning: count, scan (2), place, chunk lists, reset, counter
-            "gpu_launches": launches_per_step * args.steps + 7 * (rebins - rebins_before),
+            # 4 kernels per re-binning: count, segments, place, reset
+            "gpu_launches": launches_per_step * args.steps + 4 * (rebins - rebins_before),
             "clocks": clocks}
     return line, scenes
 

@@ -331,8 +331,8 @@ int mpm_num_kernel_configs(void);
 int mpm_kernel_config_info(int config, int *chunk, int *min_ctas, int *rounds);
 /* How a configuration orders and scatters the particles: *cell_major = 1 when
  * the re-binning puts a cell's particles together (else rank-major: a warp's
- * lanes in distinct cells); *segmented = 1 when the lanes of a warp that share
- * a stencil base are summed in shared memory before one reduction per node
+ * lanes in distinct cells); *segmented = 1 when the particles of a chunk that
+ * share a stencil base are summed before one reduction per node
  * (else every particle reduces its own 3^D node values).  The reference
  * scatters every particle's values with FP64 atomics (MPMCUDA.cu:388-421). */
 int mpm_kernel_config_scatter(int config, int *cell_major, int *segmented);

@@ -9,19 +9,22 @@
 // k_g2p2g is bound by the L1 data pipe and the L1-to-L2 request path (66 % busy
 // each on the 2M-particle jello scene): a float4 reduction instruction takes 26
 // data wavefronts, and it issues 27 per particle.  Here a run's particles share
-// its 27 reductions (39.3M -> 6.3M reduction sectors per launch; data pipe 48 %,
-// request path 25 %), for 19 % more instructions; the pass is bound by
-// instruction issue (63 % of the issue slots).  Fused pass, 128 threads x 2
-// particles against the best direct configuration: jello 256^3 2M particles 248
-// against 322 us, snow 256^3 264 against 311, jello 128^3 70 against 88, water
-// 149 x 122 x 83 600k particles 71 against 101, 16 mixed scenes 294 against 364.
+// its 27 reductions (39.3M -> 5.0M reduction requests' sectors per launch).  What
+// bounds it now: the issue rate (60 % of the slots, 16 warps an SM), the data
+// pipe (56 %: window gathers and records) and the waits at the three barriers of
+// a chunk (1.6 stall cycles per issue).  Substep, the best configuration of the
+// per-particle scatter with the decomposed stress against run sums with the
+// polar one: jello 256^3 2M particles 320 -> 203 us, snow 256^3 331 -> 217, jello
+// 128^3 450k 90 -> 54.7, water 149 x 122 x 83 600k 104 -> 64, 16 mixed scenes 376
+// -> 216, 2D water 40k 12.5 -> 9.1, paged snow 152 -> 103.  By themselves the run
+// sums took jello 256^3 from 320 to 260, snow to 300.
 // The records stay in the order of the particles: linking them per base (one
 // exchange each) needs no sort, and a drifted particle joins its new base's run.
-// Ordering the runs by length (a counting sort over 16 lengths, two barriers)
-// keeps a warp's lanes on runs of about one length: 248 -> 239 us, jello 128^3
-// 70.5 -> 67.7 us.  Letting a warp start on the next chunk before the others
-// have summed their runs (the first barrier moved to the first record) was
-// slower: the values live across it spill (213 -> 217 us with the Newton stress).
+// Ordering the runs by length (a counting sort over 16 lengths whose counts the
+// insertions keep) keeps a warp's lanes on runs of about one length: fused pass
+// 248 -> 239 us, jello 128^3 70.5 -> 67.7.  Letting a warp start on the next chunk
+// before the others have summed their runs (the first barrier moved to the first
+// record) was slower: the values live across it spill (213 -> 217 us).
 #pragma once
 
 #include "mpm_kernels_binned.cuh"
