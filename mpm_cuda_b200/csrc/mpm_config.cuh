@@ -86,6 +86,25 @@ constexpr bool sums_runs(int cfg, bool paged) {
     return paged ? c.scatter == SCATTER_DIRECT && c.order == ORDER_CELL && c.chunk == 128 && c.min_ctas <= 5
                  : c.scatter == SCATTER_RUNS;
 }
+// Material that sprays leaves chunks of a few particles, for which a CTA of a
+// run-sum configuration with several particles per thread pays its window, its
+// lists and its three barriers all the same, four or five CTAs an SM.  Such a
+// state hands the chunks of at most 64 particles to launches of kSmallCfg, the
+// per-particle scatter with ten CTAs an SM, behind (and into, pass_end) the main
+// one: 1.9M particles of colliding snow after 2500 / 3000 / 3500 substeps 364 /
+// 447 / 547 -> 331 / 371 / 470 us a substep (the per-particle scatter alone 356 /
+// 396 / 453).  While the blocks are full it costs 3-20 %
+// (jello 128^3 54.3 -> 66: the list loses its order by size), so it begins when
+// the chunks are less than half as full as they were when the configuration was
+// chosen or set, and ends when they are fuller than 0.6 of that.
+constexpr bool may_split_small(int cfg, bool paged) { return sums_runs(cfg, paged) && kFusedCfgs[cfg].rounds >= 2; }
+constexpr bool wants_split_small(bool now, float fill, float fill_at_first) {
+    return fill < (now ? 0.6f : 0.5f) * fill_at_first;
+}
+constexpr int kSmallCfg = 16;
+static_assert(kFusedCfgs[kSmallCfg].scatter == SCATTER_DIRECT && kFusedCfgs[kSmallCfg].rounds == 1 &&
+                  kFusedCfgs[kSmallCfg].chunk == 64,
+              "a particle per thread");
 // SCATTER_RUNS: float4s of a particle's source record, and the dynamic shared
 // memory of a chunk (a record and two run-list entries per particle)
 constexpr int run_rec4(int dim) { return dim == 3 ? 6 : 4; }

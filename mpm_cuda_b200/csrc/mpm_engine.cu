@@ -30,13 +30,14 @@ enum {
     CNT_CHUNKS = 0,      // large chunks per material, then small ones
     CNT_ACTIVE = 6,
     CNT_EPOCH = 7,
-    CNT_CURSOR = 8,
     CNT_FALLBACK = 11,
     CNT_REBINS = 12,
     CNT_UPDATE_DONE = 13,
     CNT_POOL_FREE = 14,  // paged grid: height of the free stack
     CNT_DET_RUNS = 15,   // deterministic P2G: number of runs of records sharing a base node
     CNT_PLACED = 16,     // re-binning: particles given a segment so far
+    CNT_CURSOR = 18,     // per material, then per material for the small chunks
+    CNT_ERR = 31,        // the error word
     CNT_N = 32
 };
 
@@ -382,8 +383,7 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     // the fixed-scene dense kernels load their windows through vel_map; a
     // driver without tensor maps leaves the run on the table-reading kernels
     if (fixed_scene && !paged && encode_vel_map() != MPM_OK) fixed_scene = false;
-    if ((rc = alloc((void**)&err_d, sizeof(unsigned), "err")) != MPM_OK) return rc;
-    if ((e = cudaMallocHost((void**)&err_h, sizeof(unsigned))) != cudaSuccess) {
+    if ((e = cudaMallocHost((void**)&err_h, CNT_N * sizeof(unsigned))) != cudaSuccess) {
         msg = std::string("mpm_create: cudaMallocHost: ") + cudaGetErrorString(e);
         return MPM_ERR_NOMEM;
     }
@@ -407,6 +407,7 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
     if ((rc = alloc((void**)&active, total_blocks * sizeof(int), "active")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&blk_epoch, total_blocks * sizeof(int), "blk_epoch")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&counters, CNT_N * sizeof(int), "counters")) != MPM_OK) return rc;
+    err_d = (unsigned*)(counters + CNT_ERR);
     if ((rc = alloc((void**)&speed_max, scenes_h.size() * sizeof(unsigned), "speed maxima")) != MPM_OK) return rc;
     if ((rc = alloc((void**)&scene_time, scenes_h.size() * sizeof(double), "scene times")) != MPM_OK) return rc;
     // per material: at most n / (particles per chunk) full chunks plus one
@@ -484,6 +485,11 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
 
 int Engine::chunk_particles() const { return kFusedCfgs[cfg].chunk * kFusedCfgs[cfg].rounds; }
 
+// most particles of a chunk that goes to the back of its list
+int Engine::small_chunk() const {
+    return split_small ? kFusedCfgs[kSmallCfg].chunk : (chunk_particles() - 1) / 2;
+}
+
 void Engine::set_config(int ci) {
     cfg = ci;
     const int dyn = fused_dyn_smem(dim, ci, paged);
@@ -506,7 +512,16 @@ void Engine::set_config(int ci) {
             per_sm = 1;
         }
         fused_ctas[mat] = num_sms * std::max(1, per_sm);
+        if (!may_split_small(ci, paged)) continue;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_fn(dim, mat, kSmallCfg, fixed_scene, paged),
+                                                          kFusedCfgs[kSmallCfg].chunk, 0) != cudaSuccess) {
+            cudaGetLastError();
+            per_sm = 1;
+        }
+        small_ctas[mat] = num_sms * std::max(1, per_sm);
     }
+    split_small = false;
+    chunk_fill = first_fill = 0.f;
     sur_occupancy();
     drop_graphs();
     grid_dirty = true;  // chunk lists depend on the chunk size
@@ -711,7 +726,7 @@ void Engine::release() {
         gp[p] = nullptr;
         ids[p] = nullptr;
     }
-    void* ptrs[] = {groups_d, scenes_d, grid_mom, grid_vel, err_d, keys, ranks,
+    void* ptrs[] = {groups_d, scenes_d, grid_mom, grid_vel, keys, ranks,
                     cell_count, seg_count, seg_start, blk_flag, active, blk_epoch, counters, chunks,
                     pos_out, det_cells, det_rows, det_slots, det_order, det_runs, det_partial,
                     sur_counts, speed_max, scene_time,
@@ -851,7 +866,7 @@ void Engine::enqueue_rebin(int from, bool in_loop) {
     note_launch_status("k_bin_segments",
                        cudaLaunchKernelEx(&lc, dim == 3 ? k_bin_segments<3> : k_bin_segments<2>,
                                           reinterpret_cast<const int4*>(seg_count), reinterpret_cast<int4*>(seg_start),
-                                          total_blocks, chunks, list_cap, bc, chunk_particles(),
+                                          total_blocks, chunks, list_cap, bc, chunk_particles(), small_chunk(),
                                           (const SceneParams*)scenes_d, (int)scenes_h.size(), err_d));
     lc.gridDim = dim3(nb);
     {
@@ -900,12 +915,13 @@ int Engine::encode_vel_map() {
     return r == CUDA_SUCCESS ? MPM_OK : MPM_ERR_UNSUPPORTED;
 }
 
-FusedArgs Engine::fused_args(int mat, bool first) {
+FusedArgs Engine::fused_args(int mat, bool first, int part) {
     FusedArgs A;
     A.chunks = chunks + mat * list_cap;
     A.n_chunks = counters + CNT_CHUNKS + mat;
     A.list_cap = (int)list_cap;
-    A.cursor = counters + CNT_CURSOR + mat;
+    A.part = part;
+    A.cursor = counters + CNT_CURSOR + mat + (part == PART_SMALL ? kMats : 0);
     A.groups = groups_d;
     A.scenes = scenes_d;
     A.n_scenes = (int)scenes_h.size();
@@ -919,7 +935,7 @@ FusedArgs Engine::fused_args(int mat, bool first) {
     A.err_word = err_d;
     A.fallback = (unsigned*)(counters + CNT_FALLBACK);
     A.speed_max = opt.adaptive_dt ? speed_max : nullptr;
-    A.rounds = kFusedCfgs[cfg].rounds;
+    A.rounds = part == PART_SMALL ? 1 : kFusedCfgs[cfg].rounds;
     A.chunk_cap = chunk_particles();
     A.defer_vc = defer_vc_now() ? 1 : 0;
     A.scene = scenes_h[0];
@@ -948,7 +964,7 @@ void Engine::enqueue_grid_update() {
                                               : k_grid_update_active<2, false, false>));
     const cudaError_t e = cudaLaunchKernelEx(&lc, k, grid_mom, grid_vel, (const int*)active, counters + CNT_ACTIVE,
                                              blk_flag, blk_epoch, (const int*)(counters + CNT_EPOCH),
-                                             (const SceneParams*)scenes_d, n_scenes, counters + CNT_CURSOR, (int)kMats,
+                                             (const SceneParams*)scenes_d, n_scenes, counters + CNT_CURSOR, 2 * kMats,
                                              (unsigned*)(counters + CNT_UPDATE_DONE), scenes_h[0],
                                              vel_linear_mode() ? 1 : 0, pages, err_d, (int)total_blocks);
     note_launch_status("k_grid_update_active", e);
@@ -958,7 +974,8 @@ void Engine::enqueue_g2p2g(int parity) {
     bool first = true;
     for (int mat = 0; mat < kMats; ++mat) {
         if (!mat_present[mat]) continue;
-        const FusedArgs A = fused_args(mat, first);
+        const bool split = split_small && !sur_kernel(mat);
+        const FusedArgs A = fused_args(mat, first, split ? PART_LARGE : PART_ALL);
         first = false;
         if (sur_kernel(mat)) {
             const SurArgs SA{&sur->weights->f, sur->meta, sur_counts};
@@ -974,6 +991,12 @@ void Engine::enqueue_g2p2g(int parity) {
             const cudaError_t e = cudaLaunchKernelEx(&lc, fused_fn(dim, mat, cfg, fixed_scene, paged), buf(parity), A);
             note_launch_status("k_g2p2g", e);
             note_launch("fused_fn");
+            if (split) {
+                const FusedArgs S = fused_args(mat, false, PART_SMALL);
+                const cudaLaunchConfig_t ls = pdl_config(small_ctas[mat], kFusedCfgs[kSmallCfg].chunk, 0, stream, &attr);
+                note_launch_status("k_g2p2g", cudaLaunchKernelEx(&ls, fused_fn(dim, mat, kSmallCfg, fixed_scene, paged),
+                                                                 buf(parity), S));
+            }
         }
     }
 }
@@ -1157,6 +1180,17 @@ int Engine::build_graph(int parity, int rebin, int count, cudaGraphExec_t* out) 
     return MPM_OK;
 }
 
+// gives the small chunks launches of their own or takes these back, as the last
+// read of the counters suggests; the next substep re-bins
+void Engine::choose_split() {
+    if (!may_split_small(cfg, paged) || chunk_fill == 0.f) return;
+    const bool want = wants_split_small(split_small, chunk_fill, first_fill);
+    if (want == split_small) return;
+    split_small = want;
+    drop_graphs();
+    steps_since_rebin = opt.rebin_interval;
+}
+
 int Engine::step(int n) {
     if (n < 0) {
         last_error = "mpm_step: negative substep count";
@@ -1222,6 +1256,7 @@ int Engine::step(int n) {
             int rc = prologue();
             if (rc != MPM_OK) return rc;
         }
+        if (n > 0) choose_split();
         // (after the prologue, whose v/C recovery reads the previous layout)
         if (n > 0) vel_lin_state = vel_linear_mode();
         const int run = opt.rebin_interval - 1;  // plain substeps between two re-binnings
@@ -1274,12 +1309,19 @@ int Engine::step(int n) {
 
 // ----------------------------------------------------------- queries --
 
-// (a page-locked word: the copy is queued behind the substeps and one wait
-// serves both)
+// (page-locked: the copy is queued behind the substeps and one wait serves both;
+// how full the chunks are comes with it)
 int Engine::read_errors(uint32_t* bits) {
-    MPM_CUDA_TRY(cudaMemcpyAsync(err_h, err_d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream), "read error word");
+    MPM_CUDA_TRY(cudaMemcpyAsync(err_h, counters, CNT_N * sizeof(unsigned), cudaMemcpyDeviceToHost, stream),
+                 "read error word");
     MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
-    *bits = *err_h;
+    *bits = err_h[CNT_ERR];
+    if (fused() && !grid_dirty) {
+        long long n_chunks = 0;
+        for (int k = 0; k < 2 * kMats; ++k) n_chunks += err_h[CNT_CHUNKS + k];
+        chunk_fill = n_chunks > 0 ? (float)n_particles / ((float)n_chunks * chunk_particles()) : 0.f;
+        if (first_fill == 0.f) first_fill = chunk_fill;
+    }
     return MPM_OK;
 }
 

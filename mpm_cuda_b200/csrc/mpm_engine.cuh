@@ -45,7 +45,7 @@ struct Engine {
     float4* grid_mom = nullptr;  // P2G accumulation (momentum, mass)
     float4* grid_vel = nullptr;  // after the grid update (velocity, mass)
     unsigned* err_d = nullptr;
-    unsigned* err_h = nullptr;  // page-locked copy of the error word
+    unsigned* err_h = nullptr;  // page-locked copy of the counters, the error word among them
 
     // binning and block activity
     // binning: (home block, material, cell) and rank in the cell of each particle;
@@ -92,6 +92,12 @@ struct Engine {
     int cfg = 1;                     // index into kFusedCfgs
     // particles per chunk of the current configuration (CTA size x rounds)
     int chunk_particles() const;
+    int small_chunk() const;
+    void choose_split();
+    bool split_small = false;  // small chunks have launches of their own (wants_split_small)
+    float chunk_fill = 0.f;    // particles per chunk over its capacity at the last read; 0: not read yet
+    float first_fill = 0.f;    // the same at the first read after set_config
+    int small_ctas[3] = {0, 0, 0};  // those of the launches for small chunks
     bool fixed_scene = false;        // one scene, fixed dt: fused kernels take it as a parameter
     // paged grid (mpm_options.grid_pool_blocks > 0): the grid arrays hold
     // pool_cap physical blocks plus the trash block; `pages` points at the
@@ -178,7 +184,7 @@ struct Engine {
     void enqueue_grid_update();
     void enqueue_adapt_dt();
     void enqueue_g2p2g(int parity);
-    FusedArgs fused_args(int mat, bool first);
+    FusedArgs fused_args(int mat, bool first, int part);
     int prologue();
     int build_graph(int parity, int rebin, int count, cudaGraphExec_t* out);
     void drop_graphs();

@@ -243,7 +243,8 @@ __device__ __forceinline__ void tile_origin(const SceneParams& sc, long long lb,
 template <int D>
 __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ seg_count, int4* __restrict__ seg_start,
                                                       long long n_blocks, Chunk* __restrict__ chunks, long long list_cap,
-                                                      BinCounters bc, int chunk, const SceneParams* __restrict__ scenes,
+                                                      BinCounters bc, int chunk, int small,
+                                                      const SceneParams* __restrict__ scenes,
                                                       int n_scenes, unsigned* __restrict__ err) {
     pdl_wait();
     pdl_trigger();
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(256) k_bin_segments(const int4* __restrict__ s
         if (c[m] == 0) continue;
         const int nch = (c[m] + chunk - 1) / chunk;
         const int rest = c[m] - (nch - 1) * chunk;  // the last one's particles
-        const int large = rest * 2 >= chunk ? nch : nch - 1;
+        const int large = rest > small ? nch : nch - 1;
         const int at = large ? atomicAdd(&bc.n_chunks[m], large) : 0;
         const int back = large < nch ? atomicAdd(&bc.n_chunks[kMats + m], 1) : 0;
         if (at + large > list_cap || back >= list_cap) {  // cannot happen with the list sized for the smallest chunk
@@ -547,10 +548,13 @@ __global__ void __launch_bounds__(256) k_grid_update_active(float4* __restrict__
 
 // ------------------------------------------------------------ G2P2G --
 
+enum : int { PART_ALL = 0, PART_LARGE = 1, PART_SMALL = 2 };
+
 struct FusedArgs {
     const Chunk* chunks;  // this material's chunk list: large ones from the front, small ones from the back
     const int* n_chunks;  // how many large ones, and kMats words on how many small ones
     int list_cap;
+    int part;             // the chunks of this launch: all, PART_LARGE or PART_SMALL
     int* cursor;          // next chunk to hand out (zeroed before every launch)
     const GroupParams* groups;
     const SceneParams* scenes;
@@ -590,7 +594,8 @@ struct FusedArgs {
 struct ChunkList {
     int large, all;
     __device__ __forceinline__ explicit ChunkList(const FusedArgs& A)
-        : large(A.n_chunks[0]), all(A.n_chunks[0] + A.n_chunks[kMats]) {}
+        : large(A.part == PART_SMALL ? 0 : A.n_chunks[0]),
+          all(large + (A.part == PART_LARGE ? 0 : A.n_chunks[kMats])) {}
     __device__ __forceinline__ const Chunk* at(const FusedArgs& A, int c) const {
         return A.chunks + (c < large ? c : A.list_cap - 1 - (c - large));
     }
