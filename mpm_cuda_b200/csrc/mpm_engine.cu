@@ -598,20 +598,20 @@ int Engine::autotune(int steps, float* best_ms) {
     if (e == cudaSuccess) e = cudaMalloc((void**)&bk_grp, cap * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc((void**)&bk_id, cap * sizeof(uint32_t));
     unsigned err_before = 0;
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) e = cudaMemcpy(&err_before, err_d, sizeof(unsigned), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(bk_state, st[cur], state_bytes, cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(bk_grp, gp[cur], cap * sizeof(uint16_t), cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(bk_id, ids[cur], cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&err_before, err_d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bk_state, st[cur], state_bytes, cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bk_grp, gp[cur], cap * sizeof(uint16_t), cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bk_id, ids[cur], cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream);
     const double t0 = current_time;
     const long long f0 = current_frame;
     // adaptive dt changes the scene table and the scene times: restore them too
     std::vector<SceneParams> bk_scenes(scenes_h.size());
     std::vector<double> bk_time(scenes_h.size());
     if (e == cudaSuccess)
-        e = cudaMemcpy(bk_scenes.data(), scenes_d, bk_scenes.size() * sizeof(SceneParams), cudaMemcpyDeviceToHost);
+        e = cudaMemcpyAsync(bk_scenes.data(), scenes_d, bk_scenes.size() * sizeof(SceneParams), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess)
-        e = cudaMemcpy(bk_time.data(), scene_time, bk_time.size() * sizeof(double), cudaMemcpyDeviceToHost);
+        e = cudaMemcpyAsync(bk_time.data(), scene_time, bk_time.size() * sizeof(double), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     const int mode0 = opt.p2g_mode;
     opt.p2g_mode = MPM_P2G_ATOMIC;
     int best = cfg;
@@ -675,16 +675,17 @@ int Engine::autotune(int steps, float* best_ms) {
     if (b) cudaEventDestroy(b);
     // restore
     cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) e = cudaMemcpy(st[cur], bk_state, state_bytes, cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(gp[cur], bk_grp, cap * sizeof(uint16_t), cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(ids[cur], bk_id, cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(err_d, &err_before, sizeof(unsigned), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(counters + CNT_FALLBACK, 0, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(st[cur], bk_state, state_bytes, cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(gp[cur], bk_grp, cap * sizeof(uint16_t), cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ids[cur], bk_id, cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(err_d, &err_before, sizeof(unsigned), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counters + CNT_FALLBACK, 0, 2 * sizeof(int), stream);
     if (e == cudaSuccess)
-        e = cudaMemcpy(scenes_d, bk_scenes.data(), bk_scenes.size() * sizeof(SceneParams), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(scenes_d, bk_scenes.data(), bk_scenes.size() * sizeof(SceneParams), cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess)
-        e = cudaMemcpy(scene_time, bk_time.data(), bk_time.size() * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(speed_max, 0, scenes_h.size() * sizeof(unsigned));
+        e = cudaMemcpyAsync(scene_time, bk_time.data(), bk_time.size() * sizeof(double), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(speed_max, 0, scenes_h.size() * sizeof(unsigned), stream);
+    cudaStreamSynchronize(stream);  // the copies have read the backups
     cudaFree(bk_state);
     cudaFree(bk_grp);
     cudaFree(bk_id);
@@ -1600,7 +1601,10 @@ int Engine::bin_stats(int64_t* fallbacks, int64_t* rebins) {
 
 // The deterministic path's buffers (source records, cells, order and run list,
 // 3^D float4 of partial sums per particle slot), allocated when the path is first
-// chosen
+// chosen.  The cells are cleared on the handle's stream, which does not wait for
+// the default stream: a clear there could still be queued behind the caller's own
+// work when the first pass counts into them (in create, which has no stream yet
+// and waits for the device, the null stream serves)
 int Engine::alloc_det() {
     if (det_partial) return MPM_OK;
     const size_t k = dim == 3 ? 27 : 9, row = dim == 3 ? SrcRow<3>::N4 : SrcRow<2>::N4;
@@ -1613,7 +1617,7 @@ int Engine::alloc_det() {
                       {(void**)&det_runs, cap * sizeof(int4)},         {(void**)&det_partial, cap * k * sizeof(float4)}};
     bool ok = true;
     for (const auto& w : want) ok = ok && cudaMalloc(w.p, w.bytes) == cudaSuccess;
-    ok = ok && cudaMemset(det_cells, 0, nodes * sizeof(int2)) == cudaSuccess;
+    ok = ok && cudaMemsetAsync(det_cells, 0, nodes * sizeof(int2), stream) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         for (const auto& w : want) {
@@ -1677,14 +1681,16 @@ int Engine::set_stress_mode(int mode, Surrogate* s) {
     MPM_CUDA_TRY(cudaSetDevice(device), "cudaSetDevice");
     MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
     if (!sur_counts) MPM_CUDA_TRY(cudaMalloc((void**)&sur_counts, 2 * sizeof(unsigned long long)), "alloc counters");
-    MPM_CUDA_TRY(cudaMemset(sur_counts, 0, 2 * sizeof(unsigned long long)), "clear counters");
+    MPM_CUDA_TRY(cudaMemsetAsync(sur_counts, 0, 2 * sizeof(unsigned long long), stream), "clear counters");
     sur = mode == MPM_STRESS_SURROGATE ? s : nullptr;
     opt.stress_mode = mode;
     // eligible groups: 3D jello (snow's exact stress reuses its plasticity
     // decomposition, so the network could only cost time there)
     for (auto& g : groups_h) g.surrogate = (sur && dim == 3 && g.type == JELLO) ? 1 : 0;
-    MPM_CUDA_TRY(cudaMemcpy(groups_d, groups_h.data(), groups_h.size() * sizeof(GroupParams), cudaMemcpyHostToDevice),
+    MPM_CUDA_TRY(cudaMemcpyAsync(groups_d, groups_h.data(), groups_h.size() * sizeof(GroupParams),
+                                 cudaMemcpyHostToDevice, stream),
                  "group upload");
+    MPM_CUDA_TRY(cudaStreamSynchronize(stream), "stream sync");
     sur_version = sur ? sur->version : -1;
     sur_occupancy();
     drop_graphs();
