@@ -111,11 +111,13 @@ MPM_HD void jacobi_rotate(float* S, float* V) {
     // approximate square root and quotient only perturb the angle: c and s
     // below form an exact rotation for any t, so orthogonality does not suffer
     // (below 1e-30 the pair counts as diagonal: keeps both operations on
-    // normal numbers)
+    // normal numbers.  Without vectors nothing takes back what an angle from a
+    // root that counts as 0 would do to the eigenvalues; with them the diagonal
+    // is of order 1, so there the difference is then 0, or rederived from V)
     const float q = fmaf(diff, diff, 4.f * spq * spq);
     const float root = q > 1e-30f ? q * rsqrtf(q) : 0.f;
     const float den = fabsf(diff) + root;
-    float t = den > 1e-30f ? fast_div(2.f * spq, den) : 0.f;
+    float t = den > 1e-30f && (VECS || root > 0.f) ? fast_div(2.f * spq, den) : 0.f;
     t = diff < 0.f ? -t : t;
     const float c = rsqrtf(fmaf(t, t, 1.f));
     const float s = t * c;

@@ -215,11 +215,14 @@ __device__ __forceinline__ void snow_clamp3(const float* Fn, const GroupParams& 
             for (int j = i; j < 3; ++j)
                 E[i * 3 + j] = E[j * 3 + i] =
                     R[i] * keep.Dr[j] + R[3 + i] * keep.Dr[3 + j] + R[6 + i] * keep.Dr[6 + j];
-        auto positive = [&](float sign, float c) {  // c I + sign E positive definite
+        // c I + sign E positive definite beyond doubt: the minors above what their
+        // roundings can be (two eigenvalues within 1e-4 of 0 leave m3 smaller)
+        auto positive = [&](float sign, float c) {
             const float a = fmaf(sign, E[0], c), d = fmaf(sign, E[4], c), f = fmaf(sign, E[8], c);
             const float m2 = a * d - E[1] * E[1];
             const float m3 = f * m2 + 2.f * sign * E[1] * E[2] * E[5] - a * E[5] * E[5] - d * E[2] * E[2];
-            return a > 0.f && m2 > 0.f && m3 > 0.f;
+            const float tr = a + d + f, e = 1e-6f * tr;
+            return tr > 0.f && a > e && m2 > e * tr && m3 > e * tr * tr;
         };
         if (positive(1.f, g.theta_c) && positive(-1.f, g.theta_s)) return;
         float W[9], e[3], h[3];
@@ -233,10 +236,14 @@ __device__ __forceinline__ void snow_clamp3(const float* Fn, const GroupParams& 
             h[k] = c - e[k];
             Je *= 1.f + c;
         }
+        if (h[0] == 0.f && h[1] == 0.f && h[2] == 0.f) return;
         const float d01 = e[0] - e[1], d12 = e[1] - e[2], d02 = e[0] - e[2];
-        const float h01 = d01 > 0.f ? __fdividef(h[0] - h[1], d01) : (h[0] != 0.f ? -1.f : 0.f);
-        const float h12 = d12 > 0.f ? __fdividef(h[1] - h[2], d12) : (h[1] != 0.f ? -1.f : 0.f);
-        const float h012 = d02 > 0.f ? __fdividef(h01 - h12, d02) : 0.f;
+        // (differences below 1e-30 count as none: the quotient's divisor is a
+        // normal number.  The last term is at most d02, but what rounding leaves
+        // of its product would grow with 1 / d02: below 1e-8 it is left out)
+        const float h01 = d01 > 1e-30f ? __fdividef(h[0] - h[1], d01) : (h[0] != 0.f ? -1.f : 0.f);
+        const float h12 = d12 > 1e-30f ? __fdividef(h[1] - h[2], d12) : (h[1] != 0.f ? -1.f : 0.f);
+        const float h012 = d02 > 1e-8f ? __fdividef(h01 - h12, d02) : 0.f;
         float H[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
