@@ -593,6 +593,7 @@ struct FusedArgs {
 // ones fill the last wave
 struct ChunkList {
     int large, all;
+    __device__ __forceinline__ ChunkList(int n_large, int n) : large(n_large), all(n) {}
     __device__ __forceinline__ explicit ChunkList(const FusedArgs& A)
         : large(A.part == PART_SMALL ? 0 : A.n_chunks[0]),
           all(large + (A.part == PART_LARGE ? 0 : A.n_chunks[kMats])) {}
@@ -976,10 +977,26 @@ struct SpeedFlush {
 // end instead, so what follows the last material finds every one finished.
 // 16 scenes of jello, snow and water: substep 233 -> 216.5 us (399 -> 368 with
 // the per-particle scatter).
+// What a later pass reads (grid velocities, pages, the scene table's dt, cursors)
+// is this substep's: the first pass's wait returns when the writes of the grid
+// update and of all before it are performed, that is in L2, and every pass behind
+// it starts after each of its CTAs has returned from that wait.  A trigger itself
+// publishes nothing, so an older line in the SM's L1 is dropped by pass_acquire
+// before the CTA's first read.  (A release by the first pass ahead of its trigger
+// would put the order into the memory model's terms; it holds the trigger back:
+// 2D water 9.1 -> 9.8 us a substep, 16 mixed scenes 217 -> 227.)
 __device__ __forceinline__ void pass_begin(const FusedArgs& A) {
     if (A.first) pdl_wait();
     pdl_trigger();  // the next pass may launch
     if (A.first && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.epoch, 1);
+}
+// one thread of a later pass, ahead of a CTA barrier (box loads read through the
+// async proxy)
+__device__ __forceinline__ void pass_acquire(const FusedArgs& A) {
+    if (A.first) return;
+    int seen;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(seen) : "l"(A.epoch) : "memory");
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
 }
 __device__ __forceinline__ void pass_end(const FusedArgs& A) {
     if (!A.first) pdl_wait();
@@ -1008,6 +1025,7 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
     const ChunkList list(A);
     const int nch = list.all;
     if (threadIdx.x == 0) {
+        pass_acquire(A);
         s_cn[0] = atomicAdd(A.cursor, 1);
         s_cn[1] = atomicAdd(A.cursor, 1);
         if constexpr (TMA) {

@@ -195,6 +195,7 @@ struct __align__(128) RunShared {
     int taken[kRunBins];              // runs of a length given a place so far
     int s27[2][27];                   // PAGED: the windows' physical blocks
     int n_runs[2];
+    int list[2];                      // large and all chunks of the launch
     unsigned touched[2];              // 3^D neighbour-block bits
     int next[2];
     unsigned speed;                   // adaptive dt: this chunk's max signal speed
@@ -260,18 +261,31 @@ __device__ __forceinline__ void run_chunks(const ParticleBuf& pb, const FusedArg
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
     }
-    // The chunk list and the particles were last written before the grid update
-    // ahead of this launch began: a CTA starts once that kernel's CTAs (or those
-    // of another material's pass) have all passed their own wait.  So the first
-    // chunk's record and positions are fetched before this kernel's wait;
-    // velocities, cursors and block flags after it.
-    const ChunkList list(A);
-    const int nch = list.all;
+    // The chunk list was last written before the grid update ahead of this launch
+    // began: a CTA starts once that kernel's CTAs (or those of another material's
+    // pass) have all passed their own wait, so its kernels' writes are in L2.  Its
+    // length and the first chunk's record are fetched from there (an SM's L1 may
+    // hold older lines until the wait) before this kernel's wait, the record ahead
+    // of knowing whether it lies at the front; everything else after the wait.  By
+    // two threads: read by all of them past L1, the length alone cost 1.4 us of
+    // the 8.8 us of a 2D water substep.
     // the first chunk is the CTA's own index, later ones come from the cursor
     int cur = blockIdx.x;
-    if (threadIdx.x == 0 && cur < nch) sm.ch[0] = *list.at(A, cur);
+    if (threadIdx.x < 2) {
+        if (threadIdx.x == 0) pass_acquire(A);
+        const int n_front = __ldcg(A.n_chunks), n_back = __ldcg(A.n_chunks + kMats);
+        const int large = A.part == PART_SMALL ? 0 : n_front, all = large + (A.part == PART_LARGE ? 0 : n_back);
+        const int4* front = reinterpret_cast<const int4*>(A.chunks + cur) + threadIdx.x;
+        int4 half = A.part != PART_SMALL && cur < A.list_cap ? __ldcg(front) : make_int4(0, 0, 0, 0);
+        if (cur >= large && cur < all)
+            half = __ldcg(reinterpret_cast<const int4*>(A.chunks + (A.list_cap - 1 - (cur - large))) + threadIdx.x);
+        reinterpret_cast<int4*>(&sm.ch[0])[threadIdx.x] = half;
+        sm.list[threadIdx.x] = threadIdx.x ? all : large;
+    }
     __syncthreads();  // the record, the barrier and the lists initialised
-    pass_begin(A);    // the grid update ahead has finished
+    const ChunkList list(sm.list[0], sm.list[1]);
+    const int nch = list.all;
+    pass_begin(A);  // the grid update ahead has finished
     if (cur < nch) load_window<D, CHUNK, FIXED, PAGED>(A, sm.ch[0], sm.tv, sm.s27[0], &sm.bar);
     cp_async_commit();
     SpeedFlush speed;
