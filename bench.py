@@ -359,6 +359,7 @@ def run_ours(args, rank, world, local_rank, dist):
     t_max_s = t_max_ms / 1e3
     value = total_particles * args.steps / t_max_s
     clocks = clk.summary()
+    _, fused_launches = sim.pass_info()
 
     # per-kernel device time (separate launches, CUDA events on the same stream)
     fallbacks, rebins = sim.bin_stats()
@@ -376,8 +377,9 @@ def run_ours(args, rank, world, local_rank, dist):
         stage_names = ["rebin", "grid_update", "g2p2g"]
         alg = {"rebin": n_part * 2 * sp, "grid_update": active_nodes * 32,
                "g2p2g": n_part * 2 * sp + active_nodes * 32}
-        # grid update + one fused kernel per material present
-        launches_per_step = 1 + len({g.material.type for sc in scenes for g in sc.groups})
+        # grid update + the fused kernels: one per material present, two while
+        # its small chunks have a launch of their own
+        launches_per_step = 1 + fused_launches
     else:
         stage_names = ["p2g", "grid_update", "g2p"]
         alg = {"p2g": n_part * sp + active_nodes * 16, "grid_update": active_nodes * 32,

@@ -333,11 +333,22 @@ int mpm_kernel_config_info(int config, int *chunk, int *min_ctas, int *rounds);
  * the re-binning puts a cell's particles together (else rank-major: a warp's
  * lanes in distinct cells); *segmented = 1 when the particles of a chunk that
  * share a stencil base are summed before one reduction per node
- * (else every particle reduces its own 3^D node values).  The reference
+ * (else every particle reduces its own 3^D node values).  *segmented holds for a
+ * dense grid; with a paged grid those configurations are refused, and the
+ * cell-major ones of 128 threads and at most 5 CTAs per SM sum instead
+ * (mpm_get_pass_info answers for a handle).  The reference
  * scatters every particle's values with FP64 atomics (MPMCUDA.cu:388-421). */
 int mpm_kernel_config_scatter(int config, int *cell_major, int *segmented);
 int mpm_get_kernel_config(mpm_handle *h, int *config);
 int mpm_set_kernel_config(mpm_handle *h, int config);
+/* The fused passes of a handle (MPM_P2G_ATOMIC) as the next substep would run
+ * them, as far as is known: *run_sums = 1 when its configuration sums the
+ * particles that share a stencil base on this handle's grid; *launches = fused
+ * kernels per substep: one per material present, two for a material whose
+ * particles have sprayed so far that small chunks have a launch of their own
+ * (decided at mpm_step from what the last synchronising call read).  Either may
+ * be NULL. */
+int mpm_get_pass_info(mpm_handle *h, int *run_sums, int *launches);
 
 /* Times n_substeps of every configuration on a copy of the state (the
  * simulation does not advance), keeps the fastest and caches it for handles

@@ -101,6 +101,7 @@ EXPORTS = {
     "mpm_kernel_config_info": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "mpm_kernel_config_scatter": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "mpm_get_kernel_config": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
+    "mpm_get_pass_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "mpm_set_kernel_config": (C.c_int, [C.c_void_p, C.c_int]),
     "mpm_autotune": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_float)]),
     "mpm_step_noalloc": (C.c_int, [C.POINTER(SceneDesc), C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_void_p]),

@@ -232,8 +232,15 @@ int mpm_set_kernel_config(mpm_handle* h, int config) {
     if (config < 0 || config >= mpm::kNumFusedCfgs)
         return fail(h, MPM_ERR_INVALID, "mpm_set_kernel_config: config %d out of range", config);
     if (h->eng.paged && mpm::kFusedCfgs[config].scatter != mpm::SCATTER_DIRECT)
-        return fail(h, MPM_ERR_UNSUPPORTED, "mpm_set_kernel_config: config %d scatters into a dense grid", config);
+        return fail(h, MPM_ERR_UNSUPPORTED, "mpm_set_kernel_config: config %d sums runs in a dense grid", config);
     h->eng.set_config(config);
+    return MPM_OK;
+}
+
+int mpm_get_pass_info(mpm_handle* h, int* run_sums, int* launches) {
+    if (!h) return fail(nullptr, MPM_ERR_INVALID, "mpm_get_pass_info: NULL handle");
+    if (run_sums) *run_sums = mpm::sums_runs(h->eng.cfg, h->eng.paged) ? 1 : 0;
+    if (launches) *launches = h->eng.fused_launches();
     return MPM_OK;
 }
 

@@ -559,7 +559,7 @@ namespace {
 struct TuneKey {
     int device, dim, mats;
     long long particles, blocks;
-    bool paged;  // a paged grid has its own kernels (and no run sums)
+    bool paged;  // a paged grid has its own kernels (sums_runs)
     bool operator<(const TuneKey& o) const {
         if (device != o.device) return device < o.device;
         if (dim != o.dim) return dim < o.dim;
@@ -646,7 +646,7 @@ int Engine::autotune(int steps, float* best_ms) {
     std::vector<float> best_of(kNumFusedCfgs, 1e30f);
     for (int it = 0; it < 2 * kNumFusedCfgs && e == cudaSuccess && rc == MPM_OK; ++it) {
         const int ci = it % kNumFusedCfgs;
-        if (paged && kFusedCfgs[ci].scatter != SCATTER_DIRECT) continue;  // the paged grid scatters directly
+        if (paged && kFusedCfgs[ci].scatter != SCATTER_DIRECT) continue;  // refused with a paged grid
         float ms = 0.f;
         if (!time_cfg(ci, steps, ms)) break;
         best_of[ci] = std::min(best_of[ci], ms);
@@ -969,6 +969,14 @@ void Engine::enqueue_grid_update() {
                                              (unsigned*)(counters + CNT_UPDATE_DONE), scenes_h[0],
                                              vel_linear_mode() ? 1 : 0, pages, err_d, (int)total_blocks);
     note_launch_status("k_grid_update_active", e);
+}
+
+// launches of one enqueue_g2p2g
+int Engine::fused_launches() const {
+    int n = 0;
+    for (int mat = 0; mat < kMats; ++mat)
+        if (mat_present[mat]) n += split_small && !sur_kernel(mat) ? 2 : 1;
+    return n;
 }
 
 void Engine::enqueue_g2p2g(int parity) {

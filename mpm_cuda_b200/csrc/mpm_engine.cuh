@@ -155,6 +155,7 @@ struct Engine {
                   const float* aux);
     int get_grid(int scene, float* mass, float* vel);
     int count_active_nodes(int scene, int64_t* n);
+    int fused_launches() const;
     int set_p2g_mode(int mode);
     int alloc_det();
     int set_stress_mode(int mode, Surrogate* s);

@@ -299,6 +299,12 @@ class Simulation:
     def set_kernel_config(self, config: int):
         self._check(self._lib.mpm_set_kernel_config(self._h, config))
 
+    def pass_info(self):
+        """(whether the configuration sums runs on this grid, fused launches per substep)."""
+        r, n = C.c_int(), C.c_int()
+        self._check(self._lib.mpm_get_pass_info(self._h, C.byref(r), C.byref(n)))
+        return bool(r.value), n.value
+
     def autotune(self, n_substeps: int = 8):
         """(chosen configuration, ms per substep); does not advance the state."""
         c, ms = C.c_int(), C.c_float()
