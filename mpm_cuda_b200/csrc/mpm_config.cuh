@@ -91,12 +91,15 @@ constexpr bool sums_runs(int cfg, bool paged) {
 // lists and its three barriers all the same, four or five CTAs an SM.  Such a
 // state hands the chunks of at most 64 particles to launches of kSmallCfg, the
 // per-particle scatter with ten CTAs an SM, behind (and into, pass_end) the main
-// one: 1.9M particles of colliding snow after 2500 / 3000 / 3500 substeps 364 /
-// 447 / 547 -> 331 / 371 / 470 us a substep (the per-particle scatter alone 356 /
-// 396 / 453).  While the blocks are full it costs 3-20 %
+// one.  1.9M particles of colliding snow, each from the same state (two particles
+// a thread, 27): after 2500 / 3000 / 3500 / 4300 substeps 377 / 462 / 565 / 717 ->
+// 328 / 384 / 453 / 559 us a substep, the best per-particle scatter alone (35)
+// 360 / 409 / 476 / 582.  While the blocks are full it costs 3-20 %
 // (jello 128^3 54.3 -> 66: the list loses its order by size), so it begins when
 // the chunks are less than half as full as they were when the configuration was
-// chosen or set, and ends when they are fuller than 0.6 of that.
+// timed (autotune; kept with its choice for handles of the same shape) or, for
+// one the caller set, when it first ran, and ends when they are fuller than 0.6
+// of that.
 constexpr bool may_split_small(int cfg, bool paged) { return sums_runs(cfg, paged) && kFusedCfgs[cfg].rounds >= 2; }
 constexpr bool wants_split_small(bool now, float fill, float fill_at_first) {
     return fill < (now ? 0.6f : 0.5f) * fill_at_first;

@@ -467,9 +467,11 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
         return MPM_ERR_CUDA;
     }
     if (opt.kernel_config < 0 && n_particles > 0) {
-        const int cached = cached_config();
+        float fill = 0.f;
+        const int cached = cached_config(&fill);
         if (cached >= 0) {
             set_config(cached);
+            first_fill = fill;
         } else {
             const int trc = autotune(8, nullptr);
             if (trc != MPM_OK) {
@@ -569,8 +571,12 @@ struct TuneKey {
         return paged < o.paged;
     }
 };
-std::map<TuneKey, int>& tune_cache() {
-    static std::map<TuneKey, int> m;
+struct Tuned {
+    int cfg;
+    float fill;  // of the chunks it was timed with (first_fill)
+};
+std::map<TuneKey, Tuned>& tune_cache() {
+    static std::map<TuneKey, Tuned> m;
     return m;
 }
 std::mutex& tune_mutex() {
@@ -659,12 +665,15 @@ int Engine::autotune(int steps, float* best_ms) {
         if (best_of[ci] < 1e30f) order.push_back(ci);
     std::sort(order.begin(), order.end(), [&](int x, int y) { return best_of[x] < best_of[y]; });
     if (order.size() > 3) order.resize(3);
-    std::vector<float> long_of(kNumFusedCfgs, 1e30f);
+    std::vector<float> long_of(kNumFusedCfgs, 1e30f), fill_of(kNumFusedCfgs, 0.f);
     for (int it = 0; it < 2 * (int)order.size() && e == cudaSuccess && rc == MPM_OK; ++it) {
         const int ci = order[it % order.size()];
         float ms = 0.f;
         if (!time_cfg(ci, 4 * steps, ms)) break;
         long_of[ci] = std::min(long_of[ci], ms / 4.f);
+        uint32_t bits = 0;
+        if ((rc = read_errors(&bits)) != MPM_OK) break;
+        fill_of[ci] = first_fill;
     }
     for (int ci : order)
         if (long_of[ci] < best_t) {
@@ -694,6 +703,7 @@ int Engine::autotune(int steps, float* best_ms) {
     current_time = t0;
     current_frame = f0;
     set_config(best);
+    first_fill = fill_of[best];
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "autotune");
     if (rc != MPM_OK) return rc;
@@ -703,16 +713,18 @@ int Engine::autotune(int steps, float* best_ms) {
     std::lock_guard<std::mutex> lk(tune_mutex());
     // the cache serves handle creation, which starts on the plain stress: a
     // choice timed with the learned stress is not kept for it
-    if (!sur) tune_cache()[TuneKey{device, dim, mats, n_particles, total_blocks, paged}] = best;
+    if (!sur) tune_cache()[TuneKey{device, dim, mats, n_particles, total_blocks, paged}] = Tuned{best, first_fill};
     return MPM_OK;
 }
 
-int Engine::cached_config() const {
+int Engine::cached_config(float* fill) const {
     int mats = 0;
     for (int m = 0; m < kMats; ++m) mats |= mat_present[m] ? (1 << m) : 0;
     std::lock_guard<std::mutex> lk(tune_mutex());
     auto it = tune_cache().find(TuneKey{device, dim, mats, n_particles, total_blocks, paged});
-    return it == tune_cache().end() ? -1 : it->second;
+    if (it == tune_cache().end()) return -1;
+    *fill = it->second.fill;
+    return it->second.cfg;
 }
 
 void Engine::release() {

@@ -96,7 +96,7 @@ struct Engine {
     void choose_split();
     bool split_small = false;  // small chunks have launches of their own (wants_split_small)
     float chunk_fill = 0.f;    // particles per chunk over its capacity at the last read; 0: not read yet
-    float first_fill = 0.f;    // the same at the first read after set_config
+    float first_fill = 0.f;    // the same when the configuration was timed, or at the first read after set_config
     int small_ctas[3] = {0, 0, 0};  // those of the launches for small chunks
     bool fixed_scene = false;        // one scene, fixed dt: fused kernels take it as a parameter
     // paged grid (mpm_options.grid_pool_blocks > 0): the grid arrays hold
@@ -169,7 +169,7 @@ struct Engine {
     int grid_pool(int64_t* capacity, int64_t* in_use);
     void set_config(int ci);
     int autotune(int steps, float* best_ms);
-    int cached_config() const;
+    int cached_config(float* fill) const;
 
    private:
     int cuda_fail(cudaError_t e, const char* what);
