@@ -352,7 +352,9 @@ int mpm_get_pass_info(mpm_handle *h, int *run_sums, int *launches);
 
 /* Times n_substeps of every configuration on a copy of the state (the
  * simulation does not advance), keeps the fastest and caches it for handles
- * of the same shape in this process.  *chosen / *ms_per_substep may be NULL. */
+ * of the same shape (device, dimension, materials, particle and block counts,
+ * dense or paged grid, one scene of fixed dt or not, re-binning interval) in
+ * this process.  *chosen / *ms_per_substep may be NULL. */
 int mpm_autotune(mpm_handle *h, int n_substeps, int *chosen, float *ms_per_substep);
 
 /* Diagnostics of the binned path: *fallbacks counts particle gathers or

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "mpm_kernels_binned.cuh"
 #include "mpm_kernels_det.cuh"
@@ -557,18 +558,19 @@ void Engine::sur_occupancy() {
 
 namespace {
 
-// autotuner results of this process, keyed by the workload's shape
+// autotuner results of this process, keyed by what selects the kernels and the
+// work they were timed on
 struct TuneKey {
     int device, dim, mats;
     long long particles, blocks;
-    bool paged;  // a paged grid has its own kernels (sums_runs)
+    bool paged;          // a paged grid has its own kernels (sums_runs)
+    bool fixed_scene;    // and so has one scene with a fixed dt
+    int rebin_interval;  // sets the share of particles outside their windows
     bool operator<(const TuneKey& o) const {
-        if (device != o.device) return device < o.device;
-        if (dim != o.dim) return dim < o.dim;
-        if (mats != o.mats) return mats < o.mats;
-        if (particles != o.particles) return particles < o.particles;
-        if (blocks != o.blocks) return blocks < o.blocks;
-        return paged < o.paged;
+        auto all = [](const TuneKey& k) {
+            return std::tie(k.device, k.dim, k.mats, k.particles, k.blocks, k.paged, k.fixed_scene, k.rebin_interval);
+        };
+        return all(*this) < all(o);
     }
 };
 struct Tuned {
@@ -582,6 +584,11 @@ std::map<TuneKey, Tuned>& tune_cache() {
 std::mutex& tune_mutex() {
     static std::mutex m;
     return m;
+}
+TuneKey key_of(const Engine& e) {
+    int mats = 0;
+    for (int m = 0; m < kMats; ++m) mats |= e.mat_present[m] ? (1 << m) : 0;
+    return TuneKey{e.device, e.dim, mats, e.n_particles, e.total_blocks, e.paged, e.fixed_scene, e.opt.rebin_interval};
 }
 
 }  // namespace
@@ -708,20 +715,16 @@ int Engine::autotune(int steps, float* best_ms) {
     if (e != cudaSuccess) return cuda_fail(e, "autotune");
     if (rc != MPM_OK) return rc;
     if (best_ms) *best_ms = best_t / steps;
-    int mats = 0;
-    for (int m = 0; m < kMats; ++m) mats |= mat_present[m] ? (1 << m) : 0;
     std::lock_guard<std::mutex> lk(tune_mutex());
     // the cache serves handle creation, which starts on the plain stress: a
     // choice timed with the learned stress is not kept for it
-    if (!sur) tune_cache()[TuneKey{device, dim, mats, n_particles, total_blocks, paged}] = Tuned{best, first_fill};
+    if (!sur) tune_cache()[key_of(*this)] = Tuned{best, first_fill};
     return MPM_OK;
 }
 
 int Engine::cached_config(float* fill) const {
-    int mats = 0;
-    for (int m = 0; m < kMats; ++m) mats |= mat_present[m] ? (1 << m) : 0;
     std::lock_guard<std::mutex> lk(tune_mutex());
-    auto it = tune_cache().find(TuneKey{device, dim, mats, n_particles, total_blocks, paged});
+    auto it = tune_cache().find(key_of(*this));
     if (it == tune_cache().end()) return -1;
     *fill = it->second.fill;
     return it->second.cfg;
