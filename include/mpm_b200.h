@@ -312,8 +312,8 @@ int mpm_last_error(mpm_handle *h, char *buf, size_t cap);
  *   MPM_P2G_ATOMIC:  rebin (time of one re-binning; they run every
  *                    rebin_interval substeps as in mpm_step), grid_update, g2p2g
  *   MPM_P2G_DIRECT:  p2g, grid_update, g2p
- *   MPM_P2G_DETERMINISTIC: grid_update, g2p, p2g (source records, sort,
- *                    partial sums, node sums)
+ *   MPM_P2G_DETERMINISTIC: grid_update, g2p (with the update and the source
+ *                    records), p2g (order of the runs, partial sums, node sums)
  * *n_written receives the number of stages written. */
 int mpm_profile_stages(mpm_handle *h, int n_substeps, float *out_ms, int n_out,
                        int *n_written);

@@ -1041,9 +1041,10 @@ void Engine::enqueue_adapt_dt() {
 
 // Deterministic P2G of the current state into grid_mom (step = false; blocks
 // marked active), or G2P and update from the velocities of the last grid update
-// and then the P2G of the result
+// and then the P2G of the result; stepped, when given, is recorded between the
+// particles' pass and the sums
 template <int D>
-void Engine::enqueue_det(bool step) {
+void Engine::enqueue_det(bool step, cudaEvent_t stepped) {
     const int n_scenes = (int)scenes_h.size();
     const DetCells dc{det_cells, keys, (unsigned long long)total_blocks * 64, ranks};
     const DetCounters cnt{counters + CNT_DET_RUNS, counters + CNT_PLACED};
@@ -1059,7 +1060,8 @@ void Engine::enqueue_det(bool step) {
             k_det_source<D><<<grid_blocks(n_particles, 128), 128, 0, stream>>>(
                 buf(cur), n_particles, groups_d, scenes_d, det_rows, dc, blk_flag, active, counters + CNT_ACTIVE, cnt,
                 err_d);
-        note_launch("k_det_source");
+        note_launch(step ? "k_det_step" : "k_det_source");
+        if (stepped) cudaEventRecord(stepped, stream);
         note_launch_status("k_det_starts", cudaLaunchKernelEx(&lc, k_det_starts, det_cells, (const int*)active, n_active,
                                                               det_runs, cnt));
         lc.gridDim = dim3(grid_blocks(n_particles, 256));
@@ -1075,6 +1077,7 @@ void Engine::enqueue_det(bool step) {
     } else if (step) {
         k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_EPOCH);
         note_launch("epoch");
+        if (stepped) cudaEventRecord(stepped, stream);
     }
     lc.gridDim = dim3(update_ctas);
     lc.blockDim = dim3(256);
@@ -1084,9 +1087,9 @@ void Engine::enqueue_det(bool step) {
     note_launch_status("k_det_reset", cudaLaunchKernelEx(&lc, k_det_reset, det_cells, (const int*)active, n_active));
 }
 
-void Engine::enqueue_det_p2g(bool step) {
-    if (dim == 3) enqueue_det<3>(step);
-    else enqueue_det<2>(step);
+void Engine::enqueue_det_p2g(bool step, cudaEvent_t stepped) {
+    if (dim == 3) enqueue_det<3>(step, stepped);
+    else enqueue_det<2>(step, stepped);
 }
 
 // grid update of the pending P2G, G2P from it, deterministic P2G of the result
@@ -1250,7 +1253,7 @@ int Engine::step(int n) {
             int rc = prologue();
             if (rc != MPM_OK) return rc;
         }
-        if (n > 0) vel_lin_state = false;  // read back by k_g2p_direct in the blocked layout
+        if (n > 0) vel_lin_state = false;  // read back by k_det_step in the blocked layout
         if (opt.use_graph) {
             if (!graphs[cur][0]) {
                 cudaGraph_t g = nullptr;
@@ -1809,22 +1812,12 @@ int Engine::profile_stages(int n, float* out_ms, int n_out, int* n_written) {
             int rc = prologue();
             if (rc != MPM_OK) return rc;
         }
-        if (n > 0) vel_lin_state = false;  // read back by k_g2p_direct in the blocked layout
-        const ParticleBuf pb = buf(cur);
+        if (n > 0) vel_lin_state = false;  // read back by k_det_step in the blocked layout
         for (int it = 0; it < n; ++it) {
             cudaEventRecord(ev[0], stream);
             enqueue_grid_update();
             cudaEventRecord(ev[1], stream);
-            if (dim == 3)
-                k_g2p_direct<3><<<grid_blocks(n_particles, bt), bt, 0, stream>>>(pb, n_particles, groups_d, scenes_d,
-                                                                                 grid_vel, err_d);
-            else
-                k_g2p_direct<2><<<grid_blocks(n_particles, bt), bt, 0, stream>>>(pb, n_particles, groups_d, scenes_d,
-                                                                                 grid_vel, err_d);
-            note_launch("k_g2p_direct");
-            k_count_rebin<<<1, 1, 0, stream>>>(counters + CNT_EPOCH);
-            cudaEventRecord(ev[2], stream);
-            enqueue_det_p2g(false);
+            enqueue_det_p2g(true, ev[2]);
             cudaEventRecord(ev[3], stream);
             cudaEventSynchronize(ev[3]);
             for (int st_i = 0; st_i < 3; ++st_i) {

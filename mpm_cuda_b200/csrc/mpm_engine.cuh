@@ -197,9 +197,9 @@ struct Engine {
     void sur_occupancy();
     int sur_chunk() const;
     int sur_refresh();
-    void enqueue_det_p2g(bool step);
+    void enqueue_det_p2g(bool step, cudaEvent_t stepped = nullptr);
     template <int D>
-    void enqueue_det(bool step);
+    void enqueue_det(bool step, cudaEvent_t stepped);
     void enqueue_det_substep();
     int canonical_order();
 };
