@@ -1022,10 +1022,12 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
     // TMA: completion of window b's loads; window b's n-th load completes
     // phase n, so chunk k waits for parity (k >> 1) & 1 of barrier k & 1
     __shared__ __align__(8) unsigned long long s_bar[2];
-    const ChunkList list(A);
-    const int nch = list.all;
+    __shared__ int s_list[2];  // large and all chunks of the launch
     if (threadIdx.x == 0) {
-        pass_acquire(A);
+        pass_acquire(A);  // the CTA's first read of what the grid update and the re-binning wrote comes after it
+        const ChunkList mine(A);
+        s_list[0] = mine.large;
+        s_list[1] = mine.all;
         s_cn[0] = atomicAdd(A.cursor, 1);
         s_cn[1] = atomicAdd(A.cursor, 1);
         if constexpr (TMA) {
@@ -1035,6 +1037,8 @@ __device__ __forceinline__ void chunk_loop(const FusedArgs& A, float4 (&tv)[2][T
         }
     }
     __syncthreads();
+    const ChunkList list(s_list[0], s_list[1]);
+    const int nch = list.all;
     int cur = s_cn[0], nxt = s_cn[1];
     __syncthreads();  // s_cn is rewritten below
     if (cur < nch) prefetch_velocity_tile<D, NT, FIXED, PAGED>(A, list.at(A, cur), tv[0], s27[0], &s_ch[0], &s_bar[0]);
