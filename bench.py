@@ -256,15 +256,15 @@ def time_substeps(sim, stream, flush, steps: int) -> float:
 def surrogate_leg(args, sim, scenes, stream, flush, plain_ms_per_step: float):
     """The learned-stress path on the same workload: deformation gradients
     harvested from a separate plain run of it (snapshots after the impact),
-    network trained on the GPU, held-out stress error against the SVD path,
+    network trained on the GPU, held-out stress error against the decomposition,
     then the same timed loop with the network stress."""
     from mpm_cuda_b200 import _lib as L
     from mpm_cuda_b200.surrogate import StressSurrogate
     from mpm_cuda_b200.train_surrogate import harvest, stress_error
     solids = [g for s in scenes for g in s.groups if g.material.type == L.JELLO]
     if scenes[0].dim != 3 or not solids:
-        return {"unavailable": "no 3D jello group in this workload (snow's exact stress reuses the "
-                               "decomposition of its plasticity clamp, so it keeps the plain path)"}
+        return {"unavailable": "no 3D jello group in this workload (snow's exact stress reuses what its "
+                               "plasticity clamp found, so it keeps the plain path)"}
     fresh, _ = build_workload(args.workload, 0, 1)
     hv = SURROGATE_HARVEST_BY_WORKLOAD.get(args.workload, SURROGATE_HARVEST)
     t0 = time.perf_counter()
@@ -310,7 +310,7 @@ def surrogate_leg(args, sim, scenes, stream, flush, plain_ms_per_step: float):
             "harvest_s": round(t1 - t0, 2), "train_s": round(t2 - t1, 3),
             "how": "BF16 MLP 10-64-64-9 (SiLU) trained on the GPU from F harvested at substeps "
                    f"{hv[0]}+{hv[1]}k (k=1..{hv[2]}) of a plain run; "
-                   "error = aggregate relative Kirchhoff stress error vs the SVD path on a later held-out "
+                   "error = aggregate relative Kirchhoff stress error vs the decomposition on a later held-out "
                    "snapshot; timed like the plain line (same K, W and L2 treatment)"}
 
 

@@ -68,8 +68,8 @@ enum mpm_p2g_mode {
 
 /* Stress evaluation modes */
 enum mpm_stress_mode {
-    MPM_STRESS_PLAIN = 0,     /* 3x3 SVD fixed-corotated stress */
-    MPM_STRESS_SURROGATE = 1  /* learned MLP stress with SVD fallback */
+    MPM_STRESS_PLAIN = 0,     /* fixed-corotated stress of F itself */
+    MPM_STRESS_SURROGATE = 1  /* learned MLP stress, the plain one as fallback */
 };
 
 /* Status codes */
@@ -398,10 +398,10 @@ int mpm_step_noalloc(const mpm_scene_desc *scene, float *state, int64_t plane_st
  * pass always takes an SVD (MPMCUDA.cu:87-134, 229-264).  A BF16 MLP
  * 10 -> 64 -> 64 -> 9 (SiLU) predicts the residual of sqrt(F F^T) beyond its
  * second-order series; the Kirchhoff stress of jello follows from it without
- * an SVD (snow's stress already reuses the decomposition of its plasticity
- * clamp and keeps the plain path).  Training and inference run on the
+ * an SVD (snow's stress already reuses what its plasticity clamp found and
+ * keeps the plain path).  Training and inference run on the
  * GPU's tensor cores; particles outside the training envelope, or whose error
- * estimate is above skew_tol, take the SVD path.
+ * estimate is above skew_tol, take the plain stress.
  * ---------------------------------------------------------------------- */
 typedef struct mpm_surrogate mpm_surrogate;
 
@@ -419,7 +419,7 @@ typedef struct mpm_surrogate_train_options {
 void mpm_surrogate_default_train_options(mpm_surrogate_train_options *opt);
 
 /* Untrained network on a device (its envelope is empty: every particle
- * falls back to the SVD until it is trained or loaded). */
+ * falls back to the plain stress until it is trained or loaded). */
 int mpm_surrogate_create(int device, uint64_t seed, mpm_surrogate **out);
 int mpm_surrogate_destroy(mpm_surrogate *s);
 
@@ -431,8 +431,8 @@ int mpm_surrogate_train(mpm_surrogate *s, const float *F_seed, int64_t n_seed,
                         const mpm_surrogate_train_options *opt, float *final_loss);
 
 /* Kirchhoff stress divided by mu of n deformation gradients F[n*9] for
- * lambda/mu = lam_over_mu: tau_pred from the network, tau_ref from the SVD
- * path; accepted[i] = 1 where the fused pass would use the network.  Any
+ * lambda/mu = lam_over_mu: tau_pred from the network, tau_ref from the
+ * decomposition of F; accepted[i] = 1 where the fused pass would use the network.  Any
  * output may be NULL. */
 int mpm_surrogate_eval(mpm_surrogate *s, const float *F, int64_t n, float lam_over_mu,
                        float *tau_pred, float *tau_ref, uint8_t *accepted);
@@ -460,7 +460,7 @@ int mpm_surrogate_load(const char *path, int device, mpm_surrogate **out);
  * snow, water and 2D scenes keep the plain stress. */
 int mpm_set_stress_mode(mpm_handle *h, int mode, mpm_surrogate *s);
 
-/* Particles whose stress came from the network / from the SVD fallback in
+/* Particles whose stress came from the network / from the plain fallback in
  * surrogate mode since the mode was set. */
 int mpm_get_stress_stats(mpm_handle *h, int64_t *surrogate, int64_t *fallback);
 

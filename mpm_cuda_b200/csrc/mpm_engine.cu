@@ -1710,8 +1710,8 @@ int Engine::set_stress_mode(int mode, Surrogate* s) {
     MPM_CUDA_TRY(cudaMemsetAsync(sur_counts, 0, 2 * sizeof(unsigned long long), stream), "clear counters");
     sur = mode == MPM_STRESS_SURROGATE ? s : nullptr;
     opt.stress_mode = mode;
-    // eligible groups: 3D jello (snow's exact stress reuses its plasticity
-    // decomposition, so the network could only cost time there)
+    // eligible groups: 3D jello (snow's exact stress reuses what its plasticity
+    // clamp found, so the network could only cost time there)
     for (auto& g : groups_h) g.surrogate = (sur && dim == 3 && g.type == JELLO) ? 1 : 0;
     MPM_CUDA_TRY(cudaMemcpyAsync(groups_d, groups_h.data(), groups_h.size() * sizeof(GroupParams),
                                  cudaMemcpyHostToDevice, stream),

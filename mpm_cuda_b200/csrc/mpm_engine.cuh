@@ -192,7 +192,7 @@ struct Engine {
     bool fused() const { return opt.p2g_mode == MPM_P2G_ATOMIC; }
     bool deterministic() const { return opt.p2g_mode == MPM_P2G_DETERMINISTIC; }
     bool direct() const { return opt.p2g_mode == MPM_P2G_DIRECT; }
-    // jello only: snow's exact stress reuses its plasticity decomposition
+    // jello only: snow's exact stress reuses what its plasticity clamp found
     bool sur_kernel(int mat) const { return sur && dim == 3 && mat == JELLO; }
     void sur_occupancy();
     int sur_chunk() const;

@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(CHUNK, MINB) k_g2p2g(ParticleBuf pb, const __g
                     // loaded after the gather, its register peak
                     const GroupParams g = particle_group<FIXED>(A, pb, i);
                     float F[D * D], Cn[D * D], v[D], aux;
-                    typename SnowKeep<D>::T esvd;  // snow: the plasticity step's decomposition, reused by the stress
+                    typename SnowKeep<D>::T esvd;  // snow: what the plasticity step found, reused by the stress
                     err |= update_and_store<D, MAT>(acc, sc, g, S, cap, i, x, v, Cn, F, aux,
                                                     MAT == SNOW ? &esvd : nullptr, A.defer_vc != 0);
                     if (A.speed_max) speed_bits = max(speed_bits, __float_as_uint(signal_speed<D, MAT>(v, g, aux)));

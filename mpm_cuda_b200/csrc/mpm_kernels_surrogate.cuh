@@ -1,9 +1,10 @@
 // Fused substep with the learned stress (MPM_STRESS_SURROGATE), 3D jello.
-// (Snow's exact stress costs no decomposition of its own: it reuses the one of
-// its plasticity clamp, so snow keeps the plain kernel.)  Same pass as
+// (Snow's exact stress comes almost free with its plasticity clamp, which leaves
+// the distance of F from its rotation behind, so snow keeps the plain kernel.)  Same pass as
 // k_g2p2g_runs (G2P, particle update, stress, run sums of the next P2G) with
 // the stress of eligible particles taken from the BF16 MLP (mpm_mlp.cuh)
-// instead of the decomposition in kirchhoff_fcr (MPMCUDA.cu:229-264):
+// instead of the polar iteration of kirchhoff_polar3 (MPMCUDA.cu:229-264
+// decomposes F):
 //   1. every thread: G2P, update, store the new state (v and C deferred as in
 //      k_g2p2g), keep x, v, C, F in its record's slot and write its network
 //      input (X = F F^T - I, J - 1) to its network row;
@@ -44,7 +45,7 @@ constexpr int sur_dyn_smem_max(int cta) {
 struct SurArgs {
     const mlp::Forward* weights;
     mlp::Meta meta;
-    unsigned long long* counts;  // [0] stresses from the network, [1] SVD fallbacks
+    unsigned long long* counts;  // [0] stresses from the network, [1] exact ones in their place
 };
 
 template <int CHUNK, int MINB, bool FIXED, bool PAGED>

@@ -219,7 +219,7 @@ class Simulation:
         self._check(self._lib.mpm_set_stress_mode(self._h, mode, surrogate.handle if surrogate else None))
 
     def stress_stats(self):
-        """(stresses from the network, SVD fallbacks) since the mode was set."""
+        """(stresses from the network, plain ones in their place) since the mode was set."""
         a, b = C.c_int64(), C.c_int64()
         self._check(self._lib.mpm_get_stress_stats(self._h, C.byref(a), C.byref(b)))
         return a.value, b.value

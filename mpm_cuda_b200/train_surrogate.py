@@ -1,6 +1,6 @@
 """Harvests deformation gradients from plain substeps of a workload, trains
 the learned stress surrogate on the GPU and reports its stress error on a
-held-out snapshot against the SVD path:
+held-out snapshot against the decomposition:
 
     python -m mpm_cuda_b200.train_surrogate --workload c1 --out net.mpmsur
 
