@@ -134,7 +134,8 @@ typedef struct mpm_scene_desc {
     double gravity[3]; /* the reference adds -9.8 to y (MPMSimulator.cpp:186) */
     int bc_type, bc_lo, bc_hi;
     double mass_eps;   /* nodes with mass <= mass_eps get zero velocity;
-                          reference DBL_EPSILON (MPMCUDA.cu:444) */
+                          reference DBL_EPSILON (MPMCUDA.cu:444).  Masses
+                          below FLT_MIN always count as none */
     int n_groups;
     const mpm_group_desc *groups;
     double ref_band;   /* > 0: the walls are the reference's position test with

@@ -249,7 +249,7 @@ int Engine::create(const mpm_scene_desc* scenes, int n_scenes, const mpm_options
             sp.bc_lo[a] = sp.bc_hi[a] = 0;
             if (a < dim) axis_walls(sp.n[a], d.h, d.origin[a], d.ref_band, d.bc_lo, d.bc_hi, sp.bc_lo[a], sp.bc_hi[a]);
         }
-        sp.mass_eps = (float)d.mass_eps;
+        sp.mass_eps = empty_node_mass(d.mass_eps);
         sp.n_blocks = (long long)sp.nb[0] * sp.nb[1] * sp.nb[2];
         sp.block_off = block_off;
         sp.node_off = block_off * 64;

@@ -7,6 +7,7 @@
 // on a few contiguous 1 KB runs.
 #pragma once
 
+#include <cfloat>
 #include <cmath>
 
 #include "mpm_types.cuh"
@@ -185,6 +186,12 @@ __device__ __forceinline__ float4 grid_node_update(float4 g, const SceneParams& 
     if (D == 2) v[2] = 0.f;
     return make_float4(v[0], v[1], v[2], m);
 }
+
+// The mass up to which a node counts as empty (host): mass_eps, and no less than
+// the largest subnormal.  Below the normal range a mass's reciprocal is infinite;
+// reductions into global memory flush such masses to zero, sums kept in registers
+// (the deterministic path) do not.
+inline float empty_node_mass(double mass_eps) { return std::fmax((float)mass_eps, std::nextafter(FLT_MIN, 0.f)); }
 
 // Wall thresholds of one axis (host): bc_lo / bc_hi as given, or, with
 // ref_band > 0, the nodes the reference's FP64 position test marks

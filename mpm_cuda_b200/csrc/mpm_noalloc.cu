@@ -255,7 +255,7 @@ extern "C" int mpm_step_noalloc(const mpm_scene_desc* scene, float* state, int64
         sc.bc_lo[a] = sc.bc_hi[a] = 0;
         if (a < dim) axis_walls(sc.n[a], d.h, d.origin[a], d.ref_band, d.bc_lo, d.bc_hi, sc.bc_lo[a], sc.bc_hi[a]);
     }
-    sc.mass_eps = (float)d.mass_eps;
+    sc.mass_eps = empty_node_mass(d.mass_eps);
     sc.node_off = 0;
     sc.block_off = 0;
 
